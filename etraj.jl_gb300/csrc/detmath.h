@@ -26,10 +26,26 @@
 #include <math.h>
 #include <string.h>
 
+#if defined(__CUDACC__) || defined(ETRAJ_DM_INT)
+#include "fpint.h"
+#endif
 #if defined(__CUDACC__)
 #define DM_FN static __host__ __device__ __forceinline__
 #else
 #define DM_FN static inline
+#endif
+
+/* On the device the divisions, square roots, series, roundings and comparisons run on
+ * the integer pipe (fpint.h), with the same results: an FP64 instruction holds its
+ * issue port for 76 cycles there, a division nine times that. */
+#if defined(__CUDA_ARCH__) || defined(ETRAJ_DM_INT) /* (ETRAJ_DM_INT: a host build of them, for tests) */
+#define DM_INT 1
+#define DM_DIV(a, b) fi_div((a), (b))
+#define DM_SQRT(a) fi_sqrt(a)
+#else
+#define DM_INT 0
+#define DM_DIV(a, b) ((a) / (b))
+#define DM_SQRT(a) sqrt(a)
 #endif
 
 /* ---- constants (mathematical values split into double parts) ---------- */
@@ -86,6 +102,9 @@ DM_FN double dm_scale(double p, int k) {
 /* Taylor series of e^r - 1 - r, divided by r^2, for |r| <= ln2/2
  * (truncation after the 1/13! term: relative error < 5e-18). */
 DM_FN double dm_expm1_tail(double r) {
+#if DM_INT
+    return fi_expm1_tail(r);
+#else
     double p = 1.0 / 6227020800.0;      /* 1/13! */
     p = fma(p, r, 1.0 / 479001600.0);   /* 1/12! */
     p = fma(p, r, 1.0 / 39916800.0);    /* 1/11! */
@@ -99,6 +118,7 @@ DM_FN double dm_expm1_tail(double r) {
     p = fma(p, r, 1.0 / 6.0);           /* 1/3!  */
     p = fma(p, r, 0.5);                 /* 1/2!  */
     return p;
+#endif
 }
 
 /* Cody-Waite reduction x = k*ln2 + r, |r| <= ~ln2/2. */
@@ -111,6 +131,15 @@ DM_FN double dm_reduce_ln2(double x, double* k) {
 }
 
 DM_FN double dm_exp(double x) {
+#if DM_INT
+    if ((fi_hi(x) & 0x7fffffffu) < 0x40862000u) { /* |x| < 708: 2^k normal, and the result */
+        int ki;
+        double kk = fi_rint_small(x * DM_LOG2E, &ki);
+        double rr = fma(-kk, DM_LN2_HI, x);
+        rr = fma(-kk, DM_LN2_LO, rr);
+        return fi_scale(1.0 + fma(rr * rr, fi_expm1_tail(rr), rr), ki);
+    }
+#endif
     if (dm_isnan(x)) return x + x;
     if (x > 709.782712893384) return dm_inf();
     if (x < -745.1332191019412) return 0.0;
@@ -121,6 +150,22 @@ DM_FN double dm_exp(double x) {
 }
 
 DM_FN double dm_expm1(double x) {
+#if DM_INT
+    if (fi_hi(x) < 0x40862000u || (fi_hi(x) ^ 0x80000000u) < 0x40430000u) { /* -38 < x < 708 */
+        int ki;
+        double kk = fi_rint_small(x * DM_LOG2E, &ki);
+        double rr = x;
+        if (ki != 0) {
+            rr = fma(-kk, DM_LN2_HI, x);
+            rr = fma(-kk, DM_LN2_LO, rr);
+        }
+        double e = fma(rr * rr, fi_expm1_tail(rr), rr);
+        if (ki == 0) return e;
+        if (ki > 1000) return fi_scale(1.0 + e, ki);
+        double t = dm_pow2i(ki);
+        return fma(t, e, t - 1.0);
+    }
+#endif
     if (dm_isnan(x)) return x + x;
     if (x > 709.782712893384) return dm_inf();
     if (x < -38.0) return -1.0;
@@ -137,6 +182,23 @@ DM_FN double dm_expm1(double x) {
 
 /* ---- log / log1p ------------------------------------------------------- */
 DM_FN double dm_log(double x) {
+#if DM_INT
+    if (fi_hi(x) - 0x00100000u < 0x7fe00000u) { /* positive, normal, finite */
+        uint64_t v = fi_bits(x);
+        int ie = (int)(v >> 52) - 1023;
+        v = (v & 0x000fffffffffffffull) | 0x3ff0000000000000ull;
+        if (v > 0x3ff6a09e667f3bcdull) { /* sqrt 2 */
+            v -= 0x0010000000000000ull;
+            ie += 1;
+        }
+        double f = fi_real(v) - 1.0;
+        double s = fi_div(f, 2.0 + f);
+        double s2 = s * s, two_s = 2.0 * s;
+        double lm = fma(two_s * s2, fi_log_poly(s2), two_s);
+        double de = fi_from_int(ie);
+        return fma(de, DM_LN2_HI, fma(de, DM_LN2_LO, lm));
+    }
+#endif
     if (dm_isnan(x)) return x + x;
     if (x < 0.0) return dm_nan();
     if (x == 0.0) return -dm_inf();
@@ -156,7 +218,7 @@ DM_FN double dm_log(double x) {
     }
     /* log(m) = 2 atanh(s), s = (m-1)/(m+1), |s| <= 0.1716 */
     double f = m - 1.0;
-    double s = f / (2.0 + f);
+    double s = DM_DIV(f, 2.0 + f);
     double s2 = s * s;
     double p = 1.0 / 23.0;
     p = fma(p, s2, 1.0 / 21.0);
@@ -180,14 +242,39 @@ DM_FN double dm_log1p(double x) {
     double u = 1.0 + x;
     if (u == 1.0) return x;
     if (u == dm_inf()) return dm_log(x);
-    return dm_log(u) * (x / (u - 1.0));
+    return dm_log(u) * DM_DIV(x, u - 1.0);
 }
 
 /* x^y for x > 0 (exp(y log x)); relative error grows like |y log x| ulp. */
 DM_FN double dm_pow_pos(double x, double y) { return dm_exp(y * dm_log(x)); }
 
 /* ---- sin / cos ----------------------------------------------------------- */
+#if DM_INT
+/* series and quadrant of dm_sincos from the reduced argument */
+DM_FN void dm_sincos_reduced(double r, int q, double* sp, double* cp) {
+    double r2 = r * r;
+    const fi_pair P = fi_sincos_poly(r2);
+    double sr = fma(r * r2, P.s, r);
+    double hr = fi_half(r2);
+    double w = 1.0 - hr;
+    double cr = w + (((1.0 - w) - hr) + (r2 * r2) * P.c);
+    const double a = (q & 1) ? cr : sr, b = (q & 1) ? sr : cr;
+    *sp = fi_real(fi_bits(a) ^ ((uint64_t)(uint32_t)(q & 2) << 62));
+    *cp = fi_real(fi_bits(b) ^ ((uint64_t)(uint32_t)((q + 1) & 2) << 62));
+}
+#endif
 DM_FN void dm_sincos(double x, double* sp, double* cp) {
+#if DM_INT
+    if ((fi_hi(x) & 0x7fffffffu) < 0x41100000u) { /* |x| < 2^18 */
+        int ki;
+        double kk = fi_rint_small(x * DM_TWO_OVER_PI, &ki);
+        double rr = fma(-kk, DM_PIO2_1, x);
+        rr = fma(-kk, DM_PIO2_2, rr);
+        rr = fma(-kk, DM_PIO2_3, rr);
+        dm_sincos_reduced(rr, ki, sp, cp);
+        return;
+    }
+#endif
     if (!(fabs(x) < dm_inf())) {
         *sp = x - x;
         *cp = x - x;
@@ -233,6 +320,20 @@ DM_FN double dm_cos(double x) { double s, c; dm_sincos(x, &s, &c); return c; }
 
 /* ---- tanh / sinh / cosh -------------------------------------------------- */
 DM_FN double dm_tanh(double x) {
+#if DM_INT
+    {
+        const uint64_t u = fi_bits(x) & 0x7fffffffffffffffull;
+        if (u > 0x7ff0000000000000ull) return x + x;
+        double t = fi_real(u);
+        if (u >= 0x4036000000000000ull) { /* 22 */
+            t = 1.0;
+        } else if (u >= 0x3e112e0be826d695ull) { /* 1e-9 */
+            double em = dm_expm1(fi_scale(t, 1));
+            t = fi_div(em, em + 2.0);
+        }
+        return copysign(t, x);
+    }
+#endif
     double a = fabs(x);
     if (dm_isnan(a)) return x + x;
     double t;
@@ -240,7 +341,7 @@ DM_FN double dm_tanh(double x) {
     else if (a < 1e-9) t = a;
     else {
         double em = dm_expm1(2.0 * a);
-        t = em / (em + 2.0);
+        t = DM_DIV(em, em + 2.0);
     }
     return copysign(t, x);
 }
@@ -250,8 +351,8 @@ DM_FN void dm_sinhcosh(double x, double* shp, double* chp) {
     double a = fabs(x);
     double em = dm_expm1(a);
     double e = em + 1.0;
-    double sh = 0.5 * (em + em / e);
-    double ch = 0.5 * (e + 1.0 / e);
+    double sh = 0.5 * (em + DM_DIV(em, e));
+    double ch = 0.5 * (e + DM_DIV(1.0, e));
     *shp = copysign(sh, x);
     *chp = ch;
 }
@@ -261,13 +362,16 @@ DM_FN double dm_atan(double x) {
     double a = fabs(x);
     if (dm_isnan(a)) return x + x;
     int inv = 0;
-    if (a > 1.0) { a = 1.0 / a; inv = 1; }
+    if (a > 1.0) { a = DM_DIV(1.0, a); inv = 1; }
     /* three half-angle steps atan(y) = 2 atan(y / (1 + sqrt(1 + y^2))) */
     double y = a;
-    y = y / (1.0 + sqrt(fma(y, y, 1.0)));
-    y = y / (1.0 + sqrt(fma(y, y, 1.0)));
-    y = y / (1.0 + sqrt(fma(y, y, 1.0)));
+    y = DM_DIV(y, 1.0 + DM_SQRT(fma(y, y, 1.0)));
+    y = DM_DIV(y, 1.0 + DM_SQRT(fma(y, y, 1.0)));
+    y = DM_DIV(y, 1.0 + DM_SQRT(fma(y, y, 1.0)));
     double y2 = y * y;
+#if DM_INT
+    double p = fi_atan_poly(y2);
+#else
     double p = -1.0 / 19.0;
     p = fma(p, y2, 1.0 / 17.0);
     p = fma(p, y2, -1.0 / 15.0);
@@ -277,6 +381,7 @@ DM_FN double dm_atan(double x) {
     p = fma(p, y2, -1.0 / 7.0);
     p = fma(p, y2, 1.0 / 5.0);
     p = fma(p, y2, -1.0 / 3.0);
+#endif
     double t = 8.0 * fma(y * y2, p, y);
     if (inv) t = (DM_PIO2_1 - t) + DM_PIO2_2;
     return copysign(t, x);
@@ -297,7 +402,7 @@ DM_FN double dm_atan2(double y, double x) {
         return copysign(t, y);
     }
     if (dm_isinf(ay)) return copysign(DM_PIO2_1, y);
-    t = dm_atan(ay / ax);
+    t = dm_atan(DM_DIV(ay, ax));
     if (x < 0.0) t = (DM_PI_1 - t) + DM_PI_2;
     return copysign(t, y);
 }
@@ -307,22 +412,22 @@ DM_FN double dm_asinh(double x) {
     if (dm_isnan(a)) return x + x;
     double r;
     if (a > 268435456.0) r = dm_log(a) + DM_LN2_HI;
-    else if (a > 2.0) r = dm_log(2.0 * a + 1.0 / (sqrt(fma(a, a, 1.0)) + a));
+    else if (a > 2.0) r = dm_log(2.0 * a + DM_DIV(1.0, DM_SQRT(fma(a, a, 1.0)) + a));
     else if (a < 3.7e-9) r = a;
     else {
         double a2 = a * a;
-        r = dm_log1p(a + a2 / (1.0 + sqrt(1.0 + a2)));
+        r = dm_log1p(a + DM_DIV(a2, 1.0 + DM_SQRT(1.0 + a2)));
     }
     return copysign(r, x);
 }
 
 DM_FN double dm_acos(double x) {
     /* acos x = atan2(sqrt((1-x)(1+x)), x) */
-    return dm_atan2(sqrt((1.0 - x) * (1.0 + x)), x);
+    return dm_atan2(DM_SQRT((1.0 - x) * (1.0 + x)), x);
 }
 
 /* hypot without scaling: the arguments here are field strengths and momenta. */
-DM_FN double dm_hypot(double x, double y) { return sqrt(x * x + y * y); }
+DM_FN double dm_hypot(double x, double y) { return DM_SQRT(x * x + y * y); }
 
 /* ---- complex arithmetic ------------------------------------------------- */
 typedef struct { double re, im; } dm_cplx;
@@ -340,11 +445,11 @@ DM_FN dm_cplx dm_cmul(dm_cplx a, dm_cplx b) {
 /* Smith's algorithm (1962). */
 DM_FN dm_cplx dm_cdiv(dm_cplx a, dm_cplx b) {
     if (fabs(b.re) >= fabs(b.im)) {
-        double r = b.im / b.re, d = b.re + b.im * r;
-        return dm_c((a.re + a.im * r) / d, (a.im - a.re * r) / d);
+        double r = DM_DIV(b.im, b.re), d = b.re + b.im * r;
+        return dm_c(DM_DIV(a.re + a.im * r, d), DM_DIV(a.im - a.re * r, d));
     } else {
-        double r = b.re / b.im, d = b.re * r + b.im;
-        return dm_c((a.re * r + a.im) / d, (a.im * r - a.re) / d);
+        double r = DM_DIV(b.re, b.im), d = b.re * r + b.im;
+        return dm_c(DM_DIV(a.re * r + a.im, d), DM_DIV(a.im * r - a.re, d));
     }
 }
 DM_FN double dm_cabs2(dm_cplx a) { return a.re * a.re + a.im * a.im; }

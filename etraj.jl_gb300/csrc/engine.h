@@ -23,6 +23,9 @@ struct DMono {
     double omega, period, F0, A0, N, cep, t_shift, ellip;
     double cphi, sphi;        // cos/sin of the azimuth
     double w2n, cN, k, Npiw;  // cos^n envelope: omega/(2N), 2/N or 1/N, 200/T, N*pi/omega
+    // high words of |t - t_shift| below which both tanh windows are exactly 1, and from
+    // which one of them is exactly 0 (cos^n envelopes)
+    uint32_t in_hi, out_hi;
     double sigma, inv_s2, inv_2s2;  // Gaussian envelope
 };
 

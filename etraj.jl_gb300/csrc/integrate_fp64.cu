@@ -49,11 +49,17 @@ __device__ __forceinline__ double d_ulp(double x) {
     if (p >= -1022) return dm_pow2i(p);
     return dm_u2d(1ull << (p + 1074));
 }
+// Julia's min and max (NaN in, NaN out), compared on the integer pipe
 __device__ __forceinline__ double jmin(double a, double b) {
-    return (a != a || b != b) ? a + b : (a < b ? a : b);
+    return (fi_isnan(a) || fi_isnan(b)) ? a + b : (fi_lt(a, b) ? a : b);
 }
 __device__ __forceinline__ double jmax(double a, double b) {
-    return (a != a || b != b) ? a + b : (a > b ? a : b);
+    return (fi_isnan(a) || fi_isnan(b)) ? a + b : (fi_lt(b, a) ? a : b);
+}
+// max(|a|, |b|), NaN if either is
+__device__ __forceinline__ double max_abs(double a, double b) {
+    const uint64_t m = 0x7fffffffffffffffull, i = fi_bits(a) & m, j = fi_bits(b) & m;
+    return fi_real(i > j ? i : j);
 }
 
 template <int N>
@@ -61,10 +67,10 @@ __device__ __forceinline__ double rms_ratio(const double* v, const double* sk) {
     double acc = 0.0;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-        double q = v[j] / sk[j];
+        double q = DM_DIV(v[j], sk[j]);
         acc = fma(q, q, acc);
     }
-    return sqrt(acc / (double)N);
+    return DM_SQRT(N == 4 ? 0.25 * acc : DM_DIV(acc, (double)N));
 }
 
 template <int DIM, int PHASE, int TGT, int N>
@@ -75,7 +81,7 @@ __device__ double initdt(const DJob& J, double t, const double* u0, const double
     for (int j = 0; j < N; ++j) sk[j] = fma(fabs(u0[j]), J.rtol, ABSTOL);
     double d0 = rms_ratio<N>(u0, sk);
     double d1 = rms_ratio<N>(f0, sk);
-    double dt0 = (d0 < 1e-5 || d1 < 1e-5) ? 1e-6 : (d0 / d1) / 100.0;
+    double dt0 = (d0 < 1e-5 || d1 < 1e-5) ? 1e-6 : DM_DIV(DM_DIV(d0, d1), 100.0);
     dt0 = jmin(dt0, dtmax);
     if (dt0 < 10.0 * 2.220446049250313e-16) return 1e-6;
 #pragma unroll
@@ -83,11 +89,11 @@ __device__ double initdt(const DJob& J, double t, const double* u0, const double
     rhs<DIM, PHASE, TGT>(J, t + dt0, u1, f1);
 #pragma unroll
     for (int j = 0; j < N; ++j) df[j] = f1[j] - f0[j];
-    double d2 = rms_ratio<N>(df, sk) / dt0;
+    double d2 = DM_DIV(rms_ratio<N>(df, sk), dt0);
     double md = jmax(d1, d2);
     double dt1;
     if (md <= 1e-15) dt1 = jmax(1e-6, dt0 * 1e-3);
-    else dt1 = dm_pow_pos(10.0, -(2.0 + dm_log(md) / DM_LN10) / 5.0);
+    else dt1 = dm_pow_pos(10.0, DM_DIV(-(2.0 + DM_DIV(dm_log(md), DM_LN10)), 5.0));
     return jmax(dtmin, jmin(jmin(100.0 * dt0, dt1), dtmax));
 }
 
@@ -122,7 +128,7 @@ __device__ int solve(const DJob& J, double t0, double tf, const double* u0, doub
     while (t < tf) {
         if (iter > 0) {
             if (!accept) {
-                dt = dt / jmin(QMIN_INV, q11 / GAMMA);
+                dt = DM_DIV(dt, jmin(QMIN_INV, DM_DIV(q11, GAMMA)));
             } else {
 #pragma unroll
                 for (int j = 0; j < N; ++j) {
@@ -142,7 +148,7 @@ __device__ int solve(const DJob& J, double t0, double tf, const double* u0, doub
         if (accept) {
             bool bad = false;
 #pragma unroll
-            for (int j = 0; j < N; ++j) bad |= (u[j] != u[j]);
+            for (int j = 0; j < N; ++j) bad |= fi_isnan(u[j]) != 0;
             if (bad) { status = 3; break; }
         }
         // stages 2..7 (perform_step! of Tsit5); every sum is built left to right
@@ -206,31 +212,30 @@ __device__ int solve(const DJob& J, double t0, double tf, const double* u0, doub
             s = fma(BT6, k6[j], s);
             s = fma(BT7, k7[j], s);
             double ut = dt * s;
-            double sc = fma(jmax(fabs(uprev[j]), fabs(u[j])), J.rtol, ABSTOL);
-            double r = ut / sc;
+            double sc = fma(max_abs(uprev[j], u[j]), J.rtol, ABSTOL);
+            double r = DM_DIV(ut, sc);
             acc = fma(r, r, acc);
         }
-        const double EEst = sqrt(acc / (double)N);
+        const double EEst = DM_SQRT(N == 4 ? 0.25 * acc : DM_DIV(acc, (double)N));
         ++attempts;
         double q;
-        if (EEst == 0.0) {
+        if (fi_iszero(EEst)) {
             q = QMAX_INV;
         } else {
             q11 = dm_pow_pos(EEst, BETA1);
-            q = q11 / dm_pow_pos(qold, BETA2);
-            q = jmax(QMAX_INV, jmin(QMIN_INV, q / GAMMA));
+            q = DM_DIV(q11, dm_pow_pos(qold, BETA2));
+            q = jmax(QMAX_INV, jmin(QMIN_INV, DM_DIV(q, GAMMA)));
         }
-        accept = (EEst <= 1.0);
+        accept = fi_bits(EEst) <= 0x3ff0000000000000ull;  // EEst <= 1 (EEst >= 0 or NaN)
         if (accept) {
-            if (q >= 1.0 && q <= 1.0) q = 1.0;
             qold = jmax(EEst, QOLDINIT);
-            double dtnew = dt / q;
+            double dtnew = DM_DIV(dt, q);
             t = (fabs(t1 - tf) < 100.0 * d_ulp(jmax(t, tf))) ? tf : t1;
             dtpropose = jmax(jmin(dtmax, dtnew), dtmin);
             if (rmin) r2min = jmin(r2min, radius2<DIM>(u));
         }
     }
-    if (rmin) *rmin = sqrt(r2min);
+    if (rmin) *rmin = DM_SQRT(r2min);
 #pragma unroll
     for (int j = 0; j < N; ++j) uout[j] = (status == 0) ? u[j] : uprev[j];
     return status;
@@ -269,24 +274,24 @@ __device__ __forceinline__ bool collect(const DJob& J, int status, const double*
         const double Z = J.target.Z;
         if (PHASE == ETRAJ_PHASE_SCTS && E > 0.0) {
             phase = phase + J.target.Ip * tr;
-            double sqrtb = 1.0 / sqrt(2.0 * E);
-            double g = sqrt(1.0 + (2.0 * E) * L2);
+            double sqrtb = DM_DIV(1.0, DM_SQRT(2.0 * E));
+            double g = DM_SQRT(1.0 + (2.0 * E) * L2);
             // the 3D reference uses x*py where x*px is meant (TrajectorySimulation.jl:463)
             double rp = (DIM == 2) ? (x * px + y * py) : ((x * py + y * py) + z * pz);
-            phase = phase - (Z * sqrtb) * (dm_log(g) + dm_asinh(rp / (g * sqrtb)));
+            phase = phase - (Z * sqrtb) * (dm_log(g) + dm_asinh(DM_DIV(rp, g * sqrtb)));
         }
         phase_out = phase;
         if (E >= 0.0) {
             ionized = true;
             wion = prob;
-            double pinf = sqrt(2.0 * E);
-            double nr = sqrt((x * x + y * y) + z * z);
+            double pinf = DM_SQRT(2.0 * E);
+            double nr = DM_SQRT((x * x + y * y) + z * z);
             double pL[3], a[3], La[3];
             cross3(pv, L, pL);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) a[i] = pL[i] - (Z * rv[i]) / nr;
+            for (int i = 0; i < 3; ++i) a[i] = pL[i] - DM_DIV(Z * rv[i], nr);
             cross3(L, a, La);
-            double fac = pinf / (1.0 + (pinf * pinf) * L2);
+            double fac = DM_DIV(pinf, 1.0 + (pinf * pinf) * L2);
 #pragma unroll
             for (int i = 0; i < 3; ++i) pin[i] = fac * (pinf * La[i] - a[i]);
             int64_t lin = 0, stride = 1;
@@ -296,7 +301,7 @@ __device__ __forceinline__ bool collect(const DJob& J, int status, const double*
                 int64_t num = J.pnum[d], ix = 1;
                 if (num > 1) {
                     double pm = J.pmax[d];
-                    double v = rint((pin[d] + pm) / J.binw[d]);
+                    double v = rint(DM_DIV(pin[d] + pm, J.binw[d]));
                     if (!(v >= 1.0 && v <= (double)num)) ok = false;
                     else ix = (int64_t)v;
                 }
@@ -308,7 +313,7 @@ __device__ __forceinline__ bool collect(const DJob& J, int status, const double*
                 if (PHASE == ETRAJ_PHASE_CTMC) {
                     cre = prob;
                 } else {
-                    double sp = sqrt(prob), sn, cs;
+                    double sp = DM_SQRT(prob), sn, cs;
                     dm_sincos(phase, &sn, &cs);
                     cre = sp * cs;
                     cim = sp * sn;

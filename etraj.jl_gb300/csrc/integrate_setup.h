@@ -36,6 +36,11 @@ inline void mono_prepare(const etraj_mono_laser& in, DMono& L) {
         L.cN = (L.kind == ETRAJ_LASER_COS4) ? 2.0 / L.N : 1.0 / L.N;
         L.k = 200.0 / L.period;
         L.Npiw = (L.N * 3.141592653589793) / L.omega;
+        // the windows are tanh(k (N pi/omega -+ t)), and dm_tanh is exactly 1 from 22 on;
+        // 0.001 covers the rounding of the argument
+        const double in = L.Npiw - 22.001 / L.k, out = L.Npiw + 22.001 / L.k;
+        L.in_hi = in > 0.0 ? (uint32_t)(dm_d2u(in) >> 32) : 0u;
+        L.out_hi = (uint32_t)(dm_d2u(out) >> 32) + 1u;
     }
 }
 

@@ -94,14 +94,14 @@ MOL_FN double mol_wigner_d_sc(int j, int mp, int m, double sh, double ch) {
         cp[i] = cp[i - 1] * ch;
         sp[i] = sp[i - 1] * sh;
     }
-    const double pref = sqrt(F[j + mp] * F[j - mp] * F[j + m] * F[j - m]);
+    const double pref = DM_SQRT(F[j + mp] * F[j - mp] * F[j + m] * F[j - m]);
     double sum = 0.0;
     for (int s = 0; s <= 2 * j; ++s) {
         const int a1 = j + m - s, a3 = mp - m + s, a4 = j - mp - s;
         if (a1 < 0 || a3 < 0 || a4 < 0) continue;
         const double den = F[a1] * F[s] * F[a3] * F[a4];
         const double sign = ((mp - m + s) & 1) ? -1.0 : 1.0;
-        sum = sum + ((sign * pref / den) * cp[2 * j + m - mp - 2 * s]) * sp[mp - m + 2 * s];
+        sum = sum + (DM_DIV(sign * pref, den) * cp[2 * j + m - mp - 2 * s]) * sp[mp - m + 2 * s];
     }
     return sum;
 }
@@ -134,7 +134,7 @@ MOL_INL void mol_rotzyz(double a, double b, double g, double R[3][3]) {
 // Euler angles (z-y'-z'') of the rotation from the field frame (F along z)
 // to the molecular frame RotZYZ(rot) (obtain_FF_MF_Euler, shared_methods.jl:31-38).
 MOL_FN void mol_euler(const double rot[3], double Fx, double Fy, double F, double* a, double* b, double* g) {
-    const double FF[3][3] = {{0.0, Fy / F, Fx / F}, {0.0, -Fx / F, Fy / F}, {1.0, 0.0, 0.0}};
+    const double FF[3][3] = {{0.0, DM_DIV(Fy, F), DM_DIV(Fx, F)}, {0.0, DM_DIV(-Fx, F), DM_DIV(Fy, F)}, {1.0, 0.0, 0.0}};
     double MF[3][3], M[3][3];
     mol_rotzyz(rot[0], rot[1], rot[2], MF);
     for (int i = 0; i < 3; ++i)
@@ -167,7 +167,7 @@ MOL_FN dm_cplx mol_sph_sum(int l, int m, dm_cplx x, dm_cplx y, dm_cplx z) {
         const double den = mol_fact(k + m) * mol_fact(k) * mol_fact(l - m - 2 * k);
         double p2 = 1.0;
         for (int i = 0; i < 2 * k + m; ++i) p2 *= 2.0;
-        const double coef = ((k & 1) ? -1.0 : 1.0) / (p2 * den);
+        const double coef = DM_DIV((k & 1) ? -1.0 : 1.0, p2 * den);
         dm_cplx t = dm_cscale(dm_cpowi(xp, k + m), coef);
         t = dm_cmul(t, dm_cpowi(xm, k));
         t = dm_cmul(t, dm_cpowi(z, l - m - 2 * k));
@@ -316,9 +316,9 @@ MOL_FN double mol_wfat_g2(int ch, int nxi_max, int m_max, int lmax, const double
 // sample only: (kappa^(|m|+2)/2/F^(|m|+1)/|m|!) (4 kappa^2/F)^(2n - 2nxi - |m| - 1).
 MOL_FN double mol_wfat_A(int e, int nxi_max, double kappa, double nstar, double F) {
     const int nxi = e % (nxi_max + 1), am = e / (nxi_max + 1);
-    const double x1 = ((mol_powi(kappa, am + 2) / 2.0) / mol_powi(F, am + 1)) / mol_fact(am);
+    const double x1 = DM_DIV(DM_DIV(mol_powi(kappa, am + 2) / 2.0, mol_powi(F, am + 1)), mol_fact(am));
     const double ex = ((2.0 * nstar - (double)(2 * nxi)) - (double)am) - 1.0;
-    const double x2 = dm_pow_pos((4.0 * (kappa * kappa)) / F, ex);
+    const double x2 = dm_pow_pos(DM_DIV(4.0 * (kappa * kappa), F), ex);
     return x1 * x2;
 }
 
@@ -329,7 +329,7 @@ MOL_FN double mol_wfat_rate(int nxi_max, int m_max, const double* g2, const doub
                             double kd, double kz, double dkdt) {
     const double k2 = kd * kd + kz * kz;
     const double X = (kappa * kappa + kd * kd) + kz * kz;
-    const double E = dm_exp(((-2.0) * (X * sqrt(X))) / (3.0 * F));
+    const double E = dm_exp(DM_DIV((-2.0) * (X * DM_SQRT(X)), 3.0 * F));
     double K[MOL_MAX_L + 1];
     for (int a = 0; a <= m_max; ++a) K[a] = mol_powi(k2, a);
     double sum = 0.0;

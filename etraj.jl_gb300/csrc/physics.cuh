@@ -28,6 +28,13 @@ __host__ __device__ __forceinline__ void window(const DMono& L, double tt, doubl
 __host__ __device__ __forceinline__ void mono_F(const DMono& L, double t, double& Fx, double& Fy) {
     double tt = t - L.t_shift;
     double sth, cth, pre, cx, cy;
+#if DM_INT
+    const uint32_t at = fi_hi(tt) & 0x7fffffffu;
+    if (L.kind != ETRAJ_LASER_GAUSSIAN && at >= L.out_hi) { // after (or before) the pulse
+        Fx = Fy = (tt != tt) ? tt : 0.0;
+        return;
+    }
+#endif
     dm_sincos(L.omega * tt + L.cep, &sth, &cth);
     if (L.kind == ETRAJ_LASER_GAUSSIAN) {
         double g = dm_exp(-(tt * tt) * L.inv_2s2);
@@ -38,9 +45,15 @@ __host__ __device__ __forceinline__ void mono_F(const DMono& L, double t, double
     } else {
         double s, c, w1, w2;
         dm_sincos(tt * L.w2n, &s, &c);
-        window(L, tt, w1, w2);
         double env = (L.kind == ETRAJ_LASER_COS4) ? (c * c) * c : c;
-        pre = ((L.F0 * env) * w1) * w2;
+        pre = L.F0 * env;
+#if DM_INT
+        if (at >= L.in_hi) // (below, both windows are 1)
+#endif
+        {
+            window(L, tt, w1, w2);
+            pre = (pre * w1) * w2;
+        }
         double b = L.cN * s;
         cx = c * sth + b * cth;
         cy = (-c) * cth + b * sth;
@@ -290,20 +303,26 @@ __host__ __device__ __forceinline__ void laser_F_dual(const DLaser& L, double t,
 // leaves every result bit-identical and saves the evaluation at large r,
 // where trajectories spend most of their steps.
 __host__ __device__ __forceinline__ double sae_exp(const DTarget& T, double b, double r) {
+#if DM_INT
+    const double br = b * r;
+    if (T.skip_ok && fi_bits(br) - 0x404e000000000001ull < 0x7ff0000000000001ull - 0x404e000000000001ull) return 0.0;
+    return dm_exp(-br);
+#else
     if (T.skip_ok && b * r > 60.0) return 0.0;
     return dm_exp(-b * r);
+#endif
 }
 
 // TargetPotential (HydrogenLikeAtom.jl:75, SAEAtom.jl:84-89)
 __host__ __device__ __forceinline__ double target_V(const DTarget& T, double x, double y, double z) {
     if (T.kind == ETRAJ_TARGET_HYDROGEN_LIKE) {
         double s = ((x * x + y * y) + z * z) + T.sc;
-        return (-T.Z) * (1.0 / sqrt(s));
+        return (-T.Z) * DM_DIV(1.0, DM_SQRT(s));
     }
-    double r = sqrt((x * x + y * y) + z * z);
+    double r = DM_SQRT((x * x + y * y) + z * z);
     double num = ((T.Z + T.a1 * sae_exp(T, T.b1, r)) + (T.a2 * r) * sae_exp(T, T.b2, r)) +
                  T.a3 * sae_exp(T, T.b3, r);
-    return -num / sqrt(r * r + T.sc);
+    return DM_DIV(-num, DM_SQRT(r * r + T.sc));
 }
 
 // ODE right-hand side (TrajectoryFunction, HydrogenLikeAtom.jl:78-159, SAEAtom.jl:98-186).
@@ -318,23 +337,23 @@ __host__ __device__ __forceinline__ void rhs(const DJob& J, double t, const doub
         double tFx, tFy, Vphase;
         if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
             double s = (x * x + y * y) + T.sc;
-            double rs = sqrt(s);
-            double f = (-T.Z) * (1.0 / (s * rs));
+            double rs = DM_SQRT(s);
+            double f = (-T.Z) * DM_DIV(1.0, s * rs);
             tFx = f * x;
             tFy = f * y;
-            Vphase = T.Z * (1.0 / rs);
+            Vphase = T.Z * DM_DIV(1.0, rs);
         } else {
-            double r = sqrt(x * x + y * y);
-            double s = r * r + T.sc, rs = sqrt(s);
+            double r = DM_SQRT(x * x + y * y);
+            double s = r * r + T.sc, rs = DM_SQRT(s);
             double e1 = sae_exp(T, T.b1, r), e2 = sae_exp(T, T.b2, r), e3 = sae_exp(T, T.b3, r);
             double br = (T.Z + (T.a1 * (1.0 + T.b1 * r)) * e1) + (T.a3 * (1.0 + T.b3 * r)) * e3;
-            double coef = -((1.0 / (s * rs)) * br + ((T.a2 * T.b2) / rs) * e2);
+            double coef = -(DM_DIV(1.0, s * rs) * br + DM_DIV(T.a2 * T.b2, rs) * e2);
             tFx = x * coef;
             tFy = y * coef;
             if (PHASE != ETRAJ_PHASE_CTMC) {
                 double num = ((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3;
                 // the 2D SCTS reference divides by r^2+sc, not its square root (SAEAtom.jl:136)
-                Vphase = (PHASE == ETRAJ_PHASE_SCTS) ? num / s : num / rs;
+                Vphase = (PHASE == ETRAJ_PHASE_SCTS) ? DM_DIV(num, s) : DM_DIV(num, rs);
             } else {
                 Vphase = 0.0;
             }
@@ -350,22 +369,22 @@ __host__ __device__ __forceinline__ void rhs(const DJob& J, double t, const doub
         double tFx, tFy, tFz, Vphase;
         if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
             double s = ((x * x + y * y) + z * z) + T.sc;
-            double rs = sqrt(s);
-            double f = (-T.Z) * (1.0 / (s * rs));
+            double rs = DM_SQRT(s);
+            double f = (-T.Z) * DM_DIV(1.0, s * rs);
             tFx = f * x;
             tFy = f * y;
             tFz = f * z;
-            Vphase = T.Z * (1.0 / rs);
+            Vphase = T.Z * DM_DIV(1.0, rs);
         } else {
-            double r = sqrt((x * x + y * y) + z * z);
-            double s = r * r + T.sc, rs = sqrt(s);
+            double r = DM_SQRT((x * x + y * y) + z * z);
+            double s = r * r + T.sc, rs = DM_SQRT(s);
             double e1 = sae_exp(T, T.b1, r), e2 = sae_exp(T, T.b2, r), e3 = sae_exp(T, T.b3, r);
             double br = (T.Z + (T.a1 * (1.0 + T.b1 * r)) * e1) + (T.a3 * (1.0 + T.b3 * r)) * e3;
-            double coef = -((1.0 / (s * rs)) * br + ((T.a2 * T.b2) / rs) * e2);
+            double coef = -(DM_DIV(1.0, s * rs) * br + DM_DIV(T.a2 * T.b2, rs) * e2);
             tFx = x * coef;
             tFy = y * coef;
             tFz = z * coef;
-            Vphase = (PHASE != ETRAJ_PHASE_CTMC) ? (((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3) / rs : 0.0;
+            Vphase = (PHASE != ETRAJ_PHASE_CTMC) ? DM_DIV(((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3, rs) : 0.0;
         }
         du[0] = px;
         du[1] = py;

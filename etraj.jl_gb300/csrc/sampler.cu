@@ -61,7 +61,7 @@ __device__ __forceinline__ double fact(int n) {
 __device__ double wigner_d(int j, int mp, int m, double beta) {
     double sh, ch;
     dm_sincos(0.5 * beta, &sh, &ch);
-    double pref = sqrt(fact(j + mp) * fact(j - mp) * fact(j + m) * fact(j - m));
+    double pref = DM_SQRT(fact(j + mp) * fact(j - mp) * fact(j + m) * fact(j - m));
     double sum = 0.0;
     for (int s = 0; s <= 2 * j; ++s) {
         int a1 = j + m - s, a3 = mp - m + s, a4 = j - mp - s;
@@ -72,7 +72,7 @@ __device__ double wigner_d(int j, int mp, int m, double beta) {
         double cpow = 1.0, spow = 1.0;
         for (int i = 0; i < pc; ++i) cpow *= ch;
         for (int i = 0; i < ps; ++i) spow *= sh;
-        sum = sum + ((sign * pref / den) * cpow) * spow;
+        sum = sum + (DM_DIV(sign * pref, den) * cpow) * spow;
     }
     return sum;
 }
@@ -108,17 +108,17 @@ __global__ void k_batch_prepare(const __grid_constant__ DJob J, const double* __
     double gamma = 0.0;
     if (J.mono) {
         const DMono& M = J.laser.m[0];
-        gamma = (M.omega * J.kappa) / (M.F0 * mono_env(M, tr));
+        gamma = DM_DIV(M.omega * J.kappa, M.F0 * mono_env(M, tr));
     }
     B.c_cc = (J.cc_base * dm_pow_pos(B.F, -J.nstar)) *
-             dm_pow_pos(1.0 + (2.0 * gamma) / 2.718281828459045, -J.nstar);
+             dm_pow_pos(1.0 + DM_DIV(2.0 * gamma, 2.718281828459045), -J.nstar);
     B.W = B.Fx * B.dFy - B.dFx * B.Fy;
-    B.ny0 = B.Fy / B.F;
-    B.ny1 = -B.Fx / B.F;
-    B.nz0 = B.Fx / B.F;
-    B.nz1 = B.Fy / B.F;
+    B.ny0 = DM_DIV(B.Fy, B.F);
+    B.ny1 = DM_DIV(-B.Fx, B.F);
+    B.nz0 = DM_DIV(B.Fx, B.F);
+    B.nz1 = B.ny0;
     // Euler angles FF -> MF (shared_methods.jl:31-38), MF = RotZYZ(phi_q, theta_q, 0)
-    double FF[3][3] = {{0.0, B.Fy / B.F, B.Fx / B.F}, {0.0, -B.Fx / B.F, B.Fy / B.F}, {1.0, 0.0, 0.0}};
+    double FF[3][3] = {{0.0, B.ny0, B.nz0}, {0.0, B.ny1, B.nz1}, {1.0, 0.0, 0.0}};
     double MF[3][3], M[3][3];
     rotzyz(J.q_phi, J.q_theta, 0.0, MF);
     for (int i = 0; i < 3; ++i)
@@ -278,13 +278,13 @@ __device__ dm_cplx pre_numerator(const DJob& J, const DBatch& B, int64_t b, dm_c
 // pdf(kd) [/ pdf(kz)].  The oracle's o_mc_point evaluates the same expressions.
 __device__ __forceinline__ void mc_gauss_point(const DJob& J, double F, double ua, double ub, double* kd0,
                                                double* kz0, double* dkdt) {
-    const double sig = sqrt(F / (2.0 * J.kappa));
-    const double r = sqrt(-2.0 * dm_log(1.0 - ua));
+    const double sig = DM_SQRT(DM_DIV(F, 2.0 * J.kappa));
+    const double r = DM_SQRT(-2.0 * dm_log(1.0 - ua));
     double sn, cs;
     dm_sincos(6.283185307179586 * ub, &sn, &cs);
     const double z1 = r * cs, z2 = r * sn;
     const double norm = sig * 2.5066282746310002;  // sigma sqrt(2 pi)
-    const double inv2s2 = 1.0 / (2.0 * (sig * sig));
+    const double inv2s2 = DM_DIV(1.0, 2.0 * (sig * sig));
     double w = J.dkdt_base;
     *kd0 = 0.0;
     *kz0 = 0.0;
@@ -337,7 +337,7 @@ k_sample(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const double* _
                 const double F = B.F;
                 kx0 = kd0 * (-B.sphi);
                 ky0 = kd0 * B.cphi;
-                const double r0 = (J.Ip + (kd0 * kd0 + kz0 * kz0) / 2.0) / F;
+                const double r0 = DM_DIV(J.Ip + (kd0 * kd0 + kz0 * kz0) / 2.0, F);
                 x0 = r0 * B.cphi;
                 y0 = r0 * B.sphi;
                 const double* tb = J.mol.tab + b * (int64_t)J.mol.stride;
@@ -355,28 +355,28 @@ k_sample(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const double* _
             double F2eff = 0.0, ti, X2, Fexp;
             bool skip = false;
             if (!spane) {
-                double r0 = (Ip + (kd0 * kd0 + kz0 * kz0) / 2.0) / F;
+                double r0 = DM_DIV(Ip + (kd0 * kd0 + kz0 * kz0) / 2.0, F);
                 x0 = r0 * B.cphi;
                 y0 = r0 * B.sphi;
-                ti = sqrt((J.kappa * J.kappa + kd0 * kd0) + kz0 * kz0) / F;
+                ti = DM_DIV(DM_SQRT((J.kappa * J.kappa + kd0 * kd0) + kz0 * kz0), F);
                 X2 = (((kx0 * kx0 + ky0 * ky0) + kz0 * kz0) + 2.0 * Ip) * (F * F);
                 Fexp = F;
             } else {
                 F2eff = F * F - (kx0 * B.dFx + ky0 * B.dFy);
                 double Xk = ((kx0 * kx0 + ky0 * ky0) + kz0 * kz0) + 2.0 * Ip;
-                double r0 = ((F / 2.0) * Xk) / F2eff;
+                double r0 = DM_DIV((F / 2.0) * Xk, F2eff);
                 x0 = r0 * B.cphi;
                 y0 = r0 * B.sphi;
-                double lim = J.mc ? (F * F) / 25.0 : (F * F) / 9.0;
+                double lim = DM_DIV(F * F, J.mc ? 25.0 : 9.0);
                 skip = (F2eff <= lim);
-                ti = sqrt(((J.kappa * J.kappa + kd0 * kd0) + kz0 * kz0) / F2eff);
+                ti = DM_SQRT(DM_DIV((J.kappa * J.kappa + kd0 * kd0) + kz0 * kz0, F2eff));
                 X2 = Xk * F2eff;
-                Fexp = sqrt(F2eff);
+                Fexp = DM_SQRT(F2eff);
             }
             if (!skip) {
                 double Xe = (kd0 * kd0 + kz0 * kz0) + 2.0 * Ip;
-                double E = dm_exp(-(Xe * sqrt(Xe)) / (3.0 * Fexp));
-                double r1 = sqrt(dkdt) * E;
+                double E = dm_exp(DM_DIV(-(Xe * DM_SQRT(Xe)), 3.0 * Fexp));
+                double r1 = DM_SQRT(dkdt) * E;
                 dm_cplx amp;
                 if (J.prefix & (ETRAJ_PREFIX_PRE | ETRAJ_PREFIX_PRECC)) {
                     dm_cplx kx, ky, kz = dm_c(kz0, 0.0);
@@ -390,19 +390,19 @@ k_sample(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const double* _
                     }
                     dm_cplx num = pre_numerator(J, B, b, kx, ky, kz);
                     double cpre = (J.prefix & ETRAJ_PREFIX_PRE) ? J.c : B.c_cc;
-                    double den = (J.e_pre == 0.5) ? sqrt(X2) : dm_pow_pos(X2, J.e_pre);
+                    double den = (J.e_pre == 0.5) ? DM_SQRT(X2) : dm_pow_pos(X2, J.e_pre);
                     dm_cplx pre = dm_cscale(num, cpre);
-                    pre = dm_c(pre.re / den, pre.im / den);
+                    pre = dm_c(DM_DIV(pre.re, den), DM_DIV(pre.im, den));
                     amp = dm_cscale(pre, r1);
                 } else {
                     amp = dm_c(r1, 0.0);
                 }
                 if (J.prefix & ETRAJ_PREFIX_JAC) {
-                    double jac = spane ? fabs(F + (sqrt(kd0 * kd0 + kz0 * kz0) / (F * F)) * B.W) : F;
-                    amp = dm_cscale(amp, sqrt(jac));
+                    double jac = spane ? fabs(F + DM_DIV(DM_SQRT(kd0 * kd0 + kz0 * kz0), F * F) * B.W) : F;
+                    amp = dm_cscale(amp, DM_SQRT(jac));
                 }
                 rate = amp.re * amp.re + amp.im * amp.im;
-                double crit = spane ? rate / dkdt : rate;
+                double crit = spane ? DM_DIV(rate, dkdt) : rate;
                 keep = (!(rate != rate) && !(crit < J.cutoff)) ? 1 : 0;
                 if (keep && J.phase != ETRAJ_PHASE_CTMC) ph = dm_carg(amp);
             }
@@ -546,8 +546,8 @@ k_sample_spa(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const doubl
         double x0 = 0.0, y0 = 0.0, kx0 = 0.0, ky0 = 0.0, rate = 0.0, ph = 0.0;
         const double tr = B.tr, Ip = J.Ip;
         if (B.F > 1e-3 && !(fabs(kd0) < 1e-4)) {
-            const double w = J.spa_omega, wF = w / B.F;
-            const double guess = dm_asinh(wF * sqrt((kd0 * kd0 + kz0 * kz0) + 2.0 * Ip)) / w;
+            const double w = J.spa_omega, wF = DM_DIV(w, B.F);
+            const double guess = DM_DIV(dm_asinh(wF * DM_SQRT((kd0 * kd0 + kz0 * kz0) + 2.0 * Ip)), w);
             spa_win W;
             spa_win_init(&W);
             const double ti = spa_solve_ti(&J.laser, &W, tr, kd0, kz0, Ip, guess);
@@ -572,7 +572,7 @@ k_sample_spa(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const doubl
                 if (ok2) {
                     const dm_cplx St = dm_cneg(Si);
                     const dm_cplx iS = dm_c(0.0 * St.re - 1.0 * St.im, 0.0 * St.im + 1.0 * St.re);
-                    dm_cplx amp = dm_cscale(dm_cexp(iS), sqrt(J.dkdt));
+                    dm_cplx amp = dm_cscale(dm_cexp(iS), DM_SQRT(J.dkdt));
                     if (J.prefix & (ETRAJ_PREFIX_PRE | ETRAJ_PREFIX_PRECC)) {
                         const dm_cplx kx = dm_c(px + Ax.re, Ax.im), ky = dm_c(py + Ay.re, Ay.im);
                         const dm_cplx num = pre_numerator(J, B, b, kx, ky, dm_c(kz0, 0.0));
@@ -581,7 +581,7 @@ k_sample_spa(const __grid_constant__ DJob J, int64_t b0, int64_t nb, const doubl
                         const dm_cplx den = spa_cpow(kF, (J.nstar + 1.0) / 2.0);
                         amp = dm_cmul(amp, dm_cdiv(dm_cscale(num, cpre), den));
                     }
-                    if (J.prefix & ETRAJ_PREFIX_JAC) amp = dm_cscale(amp, sqrt(spa_jac(&J.laser, &W, tr, kd0, kz0, Ip, wF, w)));
+                    if (J.prefix & ETRAJ_PREFIX_JAC) amp = dm_cscale(amp, DM_SQRT(spa_jac(&J.laser, &W, tr, kd0, kz0, Ip, wF, w)));
                     rate = amp.re * amp.re + amp.im * amp.im;
                     keep = (!(rate != rate) && !(rate < J.cutoff)) ? 1 : 0;
                     if (keep) {

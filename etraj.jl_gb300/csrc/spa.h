@@ -71,9 +71,9 @@ SPA_HEAVY void spa_A(const SPA_LASER_T* L, spa_win* W, dm_cplx t, dm_cplx* ax, d
 
 /* momenta of the saddle-point solution (px_, py_, SPASampler.jl:230-231) */
 DM_FN void spa_pxy(double kd, dm_cplx Ax, dm_cplx Ay, double* px, double* py) {
-    const double den = sqrt(Ax.im * Ax.im + Ay.im * Ay.im);
-    *px = (kd * Ay.im) / den - Ax.re;
-    *py = ((-kd) * Ax.im) / den - Ay.re;
+    const double den = DM_SQRT(Ax.im * Ax.im + Ay.im * Ay.im);
+    *px = DM_DIV(kd * Ay.im, den) - Ax.re;
+    *py = DM_DIV((-kd) * Ax.im, den) - Ay.re;
 }
 
 /* saddle_point_equation (SPASampler.jl:233-239) */
@@ -94,7 +94,7 @@ DM_FN double spa_dspe(const SPA_LASER_T* L, spa_win* W, double tr, double x, dou
     const double e = (rel * ax > rel) ? rel * ax : rel;
     const double f1 = spa_spe(L, W, tr, x + e, kd, kz, Ip);
     const double f0 = spa_spe(L, W, tr, x - e, kd, kz, Ip);
-    return (f1 - f0) / (2.0 * e);
+    return DM_DIV(f1 - f0, 2.0 * e);
 }
 
 /* t_i of the saddle point from the initial guess x0; returns 0 when the
@@ -123,22 +123,22 @@ SPA_HEAVY double spa_solve_ti(const SPA_LASER_T* L, spa_win* W, double tr, doubl
              * until the iteration limit, i.e. no convergence */
             return 0.0;
         }
-        const double pn = -(r / J);
+        const double pn = -DM_DIV(r, J);
         if (fabs(d * pn) <= delta) {
             p = pn;
         } else {
-            const double g = (J * r) / (d * d);
+            const double g = DM_DIV(J * r, d * d);
             const double wg = fabs(d * g);
             const double Jg = J * g;
-            const double pc = ((-(wg * wg)) / (Jg * Jg)) * g;
+            const double pc = DM_DIV(-(wg * wg), Jg * Jg) * g;
             if (fabs(d * pc) >= delta) {
-                p = g * (-delta / wg);
+                p = g * DM_DIV(-delta, wg);
             } else {
                 const double df = pn - pc;
                 const double b = 2.0 * ((d * pc) * (d * df));
                 const double a = (d * df) * (d * df);
                 const double wc = fabs(d * pc);
-                const double tau = (-b + sqrt(b * b - (4.0 * a) * (wc * wc - delta * delta))) / (2.0 * a);
+                const double tau = DM_DIV(-b + DM_SQRT(b * b - (4.0 * a) * (wc * wc - delta * delta)), 2.0 * a);
                 p = pc + tau * df;
             }
         }
@@ -146,7 +146,7 @@ SPA_HEAVY double spa_solve_ti(const SPA_LASER_T* L, spa_win* W, double tr, doubl
         x = x + p;
         const double fn = spa_spe(L, W, tr, x, kd, kz, Ip);
         const double rp = J * p + r;
-        const double rho = (r * r - fn * fn) / (r * r - rp * rp);
+        const double rho = DM_DIV(r * r - fn * fn, r * r - rp * rp);
         if (rho > eta) {
             r = fn;
             converged = (fabs(x - xold) <= 0.0) || (fabs(r) <= ftol);
@@ -361,7 +361,7 @@ DM_FN void spa_exit(const spa_quad_par* P, double ti, double* x0, double* y0, in
 SPA_HEAVY double spa_jac(const SPA_LASER_T* L, spa_win* W, double tr, double kd, double kz, double Ip,
                      double omega_over_F, double omega) {
     const double dtr = 0.01, dkd = 0.01;
-#define SPA_GUESS(k) (dm_asinh(omega_over_F * sqrt(((k) * (k) + kz * kz) + 2.0 * Ip)) / omega)
+#define SPA_GUESS(k) DM_DIV(dm_asinh(omega_over_F * DM_SQRT(((k) * (k) + kz * kz) + 2.0 * Ip)), omega)
     const double ti_tp = spa_solve_ti(L, W, tr + dtr, kd, kz, Ip, SPA_GUESS(kd));
     const double ti_tm = spa_solve_ti(L, W, tr - dtr, kd, kz, Ip, SPA_GUESS(kd));
     const double ti_kp = spa_solve_ti(L, W, tr, kd + dkd, kz, Ip, SPA_GUESS(kd + dkd));
@@ -379,7 +379,7 @@ SPA_HEAVY double spa_jac(const SPA_LASER_T* L, spa_win* W, double tr, double kd,
     spa_A(L, W, dm_c(tr, ti_km), &ax, &ay);
     spa_pxy(kd - dkd, ax, ay, &pxb, &pyb);
     const double dpxdkd = pxa - pxb, dpydkd = pya - pyb;
-    return fabs(dpxdtr * dpydkd - dpxdkd * dpydtr) / ((4.0 * dtr) * dkd);
+    return DM_DIV(fabs(dpxdtr * dpydkd - dpxdkd * dpydtr), (4.0 * dtr) * dkd);
 }
 
 /* principal z^p of a complex z and real p (Julia's Complex ^ Real: |z|^p cis(p arg z)) */
