@@ -191,11 +191,14 @@ constexpr double kSample32MinCutoff = 1e-30;
 int launch_compact(const uint8_t* flag, int64_t n, int64_t* idx, uint32_t* block_sums,
                    int64_t nblocks_cap, unsigned long long* count, cudaStream_t s);
 int64_t compact_blocks(int64_t n);
+// FP64 Tsit5 solve of the survivors; work: four counters.  Without out.final_state the
+// final states replace the initial ones in soa (a 3D z goes to out.c_im), where
+// launch_collect_fp64 reads them.
 int launch_integrate_fp64(const DJob& J, InitSoA soa, const double* t, const int64_t* idx,
-                          const unsigned long long* count, TrajOut out, int64_t max_n,
+                          const unsigned long long* count, unsigned long long* work, TrajOut out, int64_t max_n,
                           int sm_count, cudaStream_t s);
-// FP64 collection of final states written by the bulk integrator (same code as
-// the epilogue of the plain kernel).
+// FP64 collection of final states (out.final_state, or as above): key, contribution and
+// weights, and the ionized bit of the status.
 int launch_collect_fp64(const DJob& J, InitSoA soa, const double* t, const int64_t* idx,
                         const unsigned long long* count, TrajOut out, int64_t max_n, int sm_count,
                         cudaStream_t s);

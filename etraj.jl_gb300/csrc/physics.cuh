@@ -327,11 +327,10 @@ __host__ __device__ __forceinline__ double target_V(const DTarget& T, double x, 
 
 // ODE right-hand side (TrajectoryFunction, HydrogenLikeAtom.jl:78-159, SAEAtom.jl:98-186).
 // DIM: 2 or 3; PHASE: ETRAJ_PHASE_*; TGT: ETRAJ_TARGET_*.
+// Fx, Fy: the laser field at the state's time.
 template <int DIM, int PHASE, int TGT>
-__host__ __device__ __forceinline__ void rhs(const DJob& J, double t, const double* u, double* du) {
+__host__ __device__ __forceinline__ void rhs_at(const DJob& J, double Fx, double Fy, const double* u, double* du) {
     const DTarget& T = J.target;
-    double Fx, Fy;
-    laser_F(J.laser, t, Fx, Fy);
     if (DIM == 2) {
         double x = u[0], y = u[1], px = u[2], py = u[3];
         double tFx, tFy, Vphase;

@@ -192,8 +192,9 @@ int launch_integrate(etraj_ctx* ctx, const DJob& J, const InitSoA& soa, const do
     }
     if (precision != ETRAJ_PRECISION_FP32_BULK) {
         if (ev) rec(ctx, ev[0], s);
-        *launches += launch_integrate_fp64(J, soa, t, idx, count, out, max_n, ctx->sm_count, s);
+        *launches += launch_integrate_fp64(J, soa, t, idx, count, work, out, max_n, ctx->sm_count, s);
         if (ev) rec(ctx, ev[1], s);
+        *launches += launch_collect_fp64(J, soa, t, idx, count, out, max_n, ctx->sm_count, s);
         return ETRAJ_OK;
     }
     BulkParams B;
