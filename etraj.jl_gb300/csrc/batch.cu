@@ -147,7 +147,7 @@ int run_batch(etraj_ctx* ctx, const etraj_job* jobs, int n, etraj_result* res, c
         ETRAJ_TRY(tuned_bulk_launch(ctx, M, P.soa, P.t, P.idx, P.count, P.work, P.out, &launches, ctx->stage_ev + 3));
         launches += launch_collect_bulk(H[0].J, P.soa, P.t, P.idx, P.count, P.out, N, ctx->sm_count, s, d_inst, n);
         rec(ctx, ctx->stage_ev[5], s);
-        launches += launch_deposit(Jgrid, P.out, P.count, N, P.dep, P.spec_re, P.spec_im, P.mspec, P.sums, P.counters, s);
+        launches += launch_deposit(Jgrid, P.out, P.count, N, P.dep, P.spec, P.mspec, P.sums, P.counters, s);
         launches += launch_instance_reductions(P.out, P.idx, P.count, d_inst, n, d_seg, d_scr, d_isums, d_icnt, s);
         if (weights) launches += launch_weighted_sum(P.mspec, n, grid1, d_w, d_wout, s);
         rec(ctx, ctx->stage_ev[6], s);
@@ -226,10 +226,8 @@ int run_batch(etraj_ctx* ctx, const etraj_job* jobs, int n, etraj_result* res, c
         const int64_t o = (int64_t)i * grid1;
         if (res[i].momentum_spec)
             cudaMemcpyAsync(res[i].momentum_spec, P.mspec + o, (size_t)grid1 * 8, cudaMemcpyDeviceToHost, s);
-        if (res[i].amplitude && coherent) {
-            cudaMemcpy2DAsync(res[i].amplitude, 16, P.spec_re + o, 8, 8, (size_t)grid1, cudaMemcpyDeviceToHost, s);
-            cudaMemcpy2DAsync(res[i].amplitude + 1, 16, P.spec_im + o, 8, 8, (size_t)grid1, cudaMemcpyDeviceToHost, s);
-        }
+        if (res[i].amplitude && coherent)
+            cudaMemcpyAsync(res[i].amplitude, P.spec + 2 * o, (size_t)grid1 * 16, cudaMemcpyDeviceToHost, s);
     }
     if (weights) cudaMemcpyAsync(wspec, d_wout, (size_t)grid1 * 8, cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);

@@ -330,7 +330,7 @@ struct DepositScratch {
 size_t deposit_scratch_bytes(int64_t max_n);
 void deposit_scratch_carve(void* base, int64_t max_n, DepositScratch* d);
 int launch_deposit(const DJob& J, const TrajOut& out, const unsigned long long* count,
-                   int64_t max_n, DepositScratch d, double* spec_re, double* spec_im,
+                   int64_t max_n, DepositScratch d, double* spec /* grid sums, or (re, im) pairs when coherent */,
                    double* momentum_spec, double* sums /* [2]: ion, unc */,
                    Counters* counters, cudaStream_t s);
 

@@ -147,8 +147,7 @@ struct Pipeline {
     unsigned long long* count = nullptr;
     TrajOut out{};
     DepositScratch dep{};
-    double* spec_re = nullptr;
-    double* spec_im = nullptr;
+    double* spec = nullptr;  // bin sums; (re, im) pairs for QTMC and SCTS
     double* mspec = nullptr;
     double* sums = nullptr;
     Counters* counters = nullptr;

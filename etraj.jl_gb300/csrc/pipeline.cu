@@ -120,8 +120,7 @@ int alloc_outputs(etraj_ctx* ctx, const DJob& J, int64_t max_n, bool with_state,
     void* dep = nullptr;
     ETRAJ_TRY(ensure(ctx, "deposit", deposit_scratch_bytes(max_n), &dep));
     deposit_scratch_carve(dep, max_n, &P.dep);
-    ETRAJ_TRY(ensure_t(ctx, "spec_re", (size_t)J.grid, &P.spec_re));
-    ETRAJ_TRY(ensure_t(ctx, "spec_im", (size_t)J.grid, &P.spec_im));
+    ETRAJ_TRY(ensure_t(ctx, "spec", (size_t)J.grid * (J.phase != ETRAJ_PHASE_CTMC ? 2 : 1), &P.spec));
     ETRAJ_TRY(ensure_t(ctx, "mspec", (size_t)J.grid, &P.mspec));
     ETRAJ_TRY(ensure_t(ctx, "sums", 2, &P.sums));
     ETRAJ_TRY(ensure_t(ctx, "counters", 1, &P.counters));
@@ -359,7 +358,7 @@ int enqueue_kernels(etraj_ctx* ctx, const etraj_job* job, const HostJob& H, cons
     ETRAJ_TRY(launch_integrate(ctx, J, P.soa, P.t, P.idx, P.count, P.out, J.n_total, P.work, job->precision,
                                H.t.front(), &launches, ctx->stage_ev + 3));
     rec(ctx, ctx->stage_ev[5], s);
-    launches += launch_deposit(J, P.out, P.count, J.n_total, P.dep, P.spec_re, P.spec_im, P.mspec, P.sums,
+    launches += launch_deposit(J, P.out, P.count, J.n_total, P.dep, P.spec, P.mspec, P.sums,
                                P.counters, s);
     rec(ctx, ctx->stage_ev[6], s);
     ctx->stage_valid = true;
@@ -505,12 +504,7 @@ int enqueue_job(etraj_ctx* ctx, const etraj_job* job, JobRec& r) {
     cudaMemcpyAsync(dst_sums, P.sums, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(dst_cnt, P.counters, sizeof(Counters), cudaMemcpyDeviceToHost, s);
     if (dst_spec) cudaMemcpyAsync(dst_spec, P.mspec, (size_t)J.grid * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (dst_amp) {
-        cudaMemcpy2DAsync(dst_amp, 2 * sizeof(double), P.spec_re, sizeof(double), sizeof(double), (size_t)J.grid,
-                          cudaMemcpyDeviceToHost, s);
-        cudaMemcpy2DAsync(dst_amp + 1, 2 * sizeof(double), P.spec_im, sizeof(double), sizeof(double), (size_t)J.grid,
-                          cudaMemcpyDeviceToHost, s);
-    }
+    if (dst_amp) cudaMemcpyAsync(dst_amp, P.spec, (size_t)J.grid * 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaEventRecord(r.ev_done, s);
     r.launches = launches;
     cudaError_t e = cudaGetLastError();

@@ -446,7 +446,7 @@ def perform_traj_simulation(*, init_cond_method, laser, target, dimension, sampl
     if dimension == 3:
         out["pz"] = _axis(final_p_max[2], final_p_num[2])
     if amp is not None:
-        out["amplitude"] = (amp[0::2] + 1j * amp[1::2]).reshape(shape, order="F")
+        out["amplitude"] = amp.view(np.complex128).reshape(shape, order="F")  # (re, im) pairs
     path = None
     if output_path:
         import os
