@@ -331,71 +331,45 @@ __host__ __device__ __forceinline__ double target_V(const DTarget& T, double x, 
 template <int DIM, int PHASE, int TGT>
 __host__ __device__ __forceinline__ void rhs_at(const DJob& J, double Fx, double Fy, const double* u, double* du) {
     const DTarget& T = J.target;
-    if (DIM == 2) {
-        double x = u[0], y = u[1], px = u[2], py = u[3];
-        double tFx, tFy, Vphase;
-        if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
-            double s = (x * x + y * y) + T.sc;
-            double rs = DM_SQRT(s);
-            double f = (-T.Z) * DM_DIV(1.0, s * rs);
-            tFx = f * x;
-            tFy = f * y;
-            Vphase = T.Z * DM_DIV(1.0, rs);
-        } else {
-            double r = DM_SQRT(x * x + y * y);
-            double s = r * r + T.sc, rs = DM_SQRT(s);
-            double e1 = sae_exp(T, T.b1, r), e2 = sae_exp(T, T.b2, r), e3 = sae_exp(T, T.b3, r);
-            double br = (T.Z + (T.a1 * (1.0 + T.b1 * r)) * e1) + (T.a3 * (1.0 + T.b3 * r)) * e3;
-            double coef = -(DM_DIV(1.0, s * rs) * br + DM_DIV(T.a2 * T.b2, rs) * e2);
-            tFx = x * coef;
-            tFy = y * coef;
-            if (PHASE != ETRAJ_PHASE_CTMC) {
-                double num = ((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3;
-                // the 2D SCTS reference divides by r^2+sc, not its square root (SAEAtom.jl:136)
-                Vphase = (PHASE == ETRAJ_PHASE_SCTS) ? DM_DIV(num, s) : DM_DIV(num, rs);
-            } else {
-                Vphase = 0.0;
-            }
-        }
-        du[0] = px;
-        du[1] = py;
-        du[2] = tFx - Fx;
-        du[3] = tFy - Fy;
-        if (PHASE == ETRAJ_PHASE_QTMC) du[4] = -((T.Ip + (px * px + py * py) / 2.0) - Vphase);
-        if (PHASE == ETRAJ_PHASE_SCTS) du[4] = -(((px * px + py * py) / 2.0 - Vphase) + (x * tFx + y * tFy));
+    const double x = u[0], y = u[1], z = (DIM == 3) ? u[2] : 0.0;
+    const double px = u[DIM], py = u[DIM + 1], pz = (DIM == 3) ? u[5] : 0.0;
+    double s = x * x + y * y;
+    if (DIM == 3) s = s + z * z;
+    double coef, Vphase = 0.0;
+    if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
+        s = s + T.sc;
+        const double rs = DM_SQRT(s);
+        coef = (-T.Z) * DM_DIV(1.0, s * rs);
+        // (the divisions are calls, which the compiler does not drop where they are not used)
+        if (PHASE != ETRAJ_PHASE_CTMC) Vphase = T.Z * DM_DIV(1.0, rs);
     } else {
-        double x = u[0], y = u[1], z = u[2], px = u[3], py = u[4], pz = u[5];
-        double tFx, tFy, tFz, Vphase;
-        if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
-            double s = ((x * x + y * y) + z * z) + T.sc;
-            double rs = DM_SQRT(s);
-            double f = (-T.Z) * DM_DIV(1.0, s * rs);
-            tFx = f * x;
-            tFy = f * y;
-            tFz = f * z;
-            Vphase = T.Z * DM_DIV(1.0, rs);
-        } else {
-            double r = DM_SQRT((x * x + y * y) + z * z);
-            double s = r * r + T.sc, rs = DM_SQRT(s);
-            double e1 = sae_exp(T, T.b1, r), e2 = sae_exp(T, T.b2, r), e3 = sae_exp(T, T.b3, r);
-            double br = (T.Z + (T.a1 * (1.0 + T.b1 * r)) * e1) + (T.a3 * (1.0 + T.b3 * r)) * e3;
-            double coef = -(DM_DIV(1.0, s * rs) * br + DM_DIV(T.a2 * T.b2, rs) * e2);
-            tFx = x * coef;
-            tFy = y * coef;
-            tFz = z * coef;
-            Vphase = (PHASE != ETRAJ_PHASE_CTMC) ? DM_DIV(((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3, rs) : 0.0;
-        }
-        du[0] = px;
-        du[1] = py;
-        du[2] = pz;
-        du[3] = tFx - Fx;
-        du[4] = tFy - Fy;
-        du[5] = tFz;
+        const double r = DM_SQRT(s);
+        s = r * r + T.sc;
+        const double rs = DM_SQRT(s);
+        const double e1 = sae_exp(T, T.b1, r), e2 = sae_exp(T, T.b2, r), e3 = sae_exp(T, T.b3, r);
+        const double br = (T.Z + (T.a1 * (1.0 + T.b1 * r)) * e1) + (T.a3 * (1.0 + T.b3 * r)) * e3;
+        coef = -(DM_DIV(1.0, s * rs) * br + DM_DIV(T.a2 * T.b2, rs) * e2);
         if (PHASE != ETRAJ_PHASE_CTMC) {
-            double K = ((px * px + py * py) + pz * pz) / 2.0;
-            if (PHASE == ETRAJ_PHASE_QTMC) du[6] = -((T.Ip + K) - Vphase);
-            else du[6] = -((K - Vphase) + ((x * tFx + y * tFy) + z * tFz));
+            const double num = ((T.Z + T.a1 * e1) + (T.a2 * r) * e2) + T.a3 * e3;
+            // the 2D SCTS reference divides by r^2+sc, not its square root (SAEAtom.jl:136)
+            Vphase = DM_DIV(num, (DIM == 2 && PHASE == ETRAJ_PHASE_SCTS) ? s : rs);
         }
+    }
+    const double tFx = coef * x, tFy = coef * y, tFz = coef * z;
+    du[0] = px;
+    du[1] = py;
+    if (DIM == 3) du[2] = pz;
+    du[DIM] = tFx - Fx;
+    du[DIM + 1] = tFy - Fy;
+    if (DIM == 3) du[5] = tFz;
+    if (PHASE != ETRAJ_PHASE_CTMC) {
+        double K = px * px + py * py, W = x * tFx + y * tFy;
+        if (DIM == 3) {
+            K = K + pz * pz;
+            W = W + z * tFz;
+        }
+        K = K / 2.0;
+        du[2 * DIM] = (PHASE == ETRAJ_PHASE_QTMC) ? -((T.Ip + K) - Vphase) : -((K - Vphase) + W);
     }
 }
 
