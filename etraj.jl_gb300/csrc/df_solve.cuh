@@ -702,6 +702,46 @@ DFS_HD void target_eval(const DFParams& P, const float* exptab, const Lane<DIM, 
     }
 }
 
+// The controller after an attempt's error estimate: acceptance (L.accept) and the next
+// step proposed.  Returns 4 (DtNaN) or 0.
+template <int DIM, int PHASE>
+DFS_HD int decide(Lane<DIM, PHASE>& L, const DFParams& P, const Tabs& T, df EEst) {
+    ++L.attempts;
+    if (!(EEst.hi == EEst.hi)) return 4;
+    L.accept = !df_lt(df_f(1.0f), EEst);
+    // log2 EEst (EEst below 1e-30 gives the same clamped q as its exact value)
+    const df l2e = df_log2(df_max(EEst, df_f(1e-30f)), T.log2c, T.rcpc);
+    if (!L.accept) {
+        L.q11 = df_exp2(df_mul(dfc(kBeta1), l2e), T.exp2);
+        return 0;
+    }
+    df q;
+    if (EEst.hi == 0.0f) {
+        q = dfc(kQmaxInv);
+    } else {
+        // q = EEst^beta1 / qold^beta2 / gamma, clamped to [1/qmax, 1/qmin]
+        q = df_exp2(df_sub(df_mul(dfc(kBeta1), l2e), df_mul(dfc(kBeta2), L.lqold)), T.exp2);
+        q = df_max(dfc(kQmaxInv), df_min(dfc(kQminInv), df_div(q, dfc(kGamma))));
+    }
+    L.lqold = df_lt(EEst, dfc(kQoldInit)) ? dfc(kLog2QoldInit) : l2e;
+    L.elast = EEst.hi;
+    L.dtprop = df_max(df_min(L.dtmax, df_div(L.dt, q)), df_f(L.dtmin));
+    return 0;
+}
+
+// The clock after an accepted step whose new state is `bad` (not a number): -1 at t_final,
+// 3 Unstable, else 0.
+template <int DIM, int PHASE>
+DFS_HD int arrive(Lane<DIM, PHASE>& L, const DFParams& P, bool bad) {
+    L.tn = L.n1;
+    L.tfr = L.f1;
+    if (L.last) return -1;
+    // within 100 ulp of t_final the FP64 solve takes t = t_final and stops
+    const df rem = df_mul(df_add(df_f((float)(P.nf - L.tn)), df_sub(d2(P.ff), L.tfr)), d2(P.h));
+    if (rem.hi < P.t_snap) return -1;
+    return bad ? 3 : 0;
+}
+
 // After the evaluation of stage 6 (slot 6): error estimate, controller and the
 // decision (the bottom of solve()'s loop).  Returns -1 when t_final is reached, a
 // status > 0 on failure (3 Unstable, 4 DtNaN), 0 to go on; after an accepted step
@@ -753,27 +793,8 @@ DFS_HD int epilogue(Lane<DIM, PHASE>& L, const DFParams& P, const Slots<KW>& k, 
         const df rf = df_div(df_mul(L.dt, ef.get()), scf);
         acc = df_fma(rf, rf, acc);
     }
-    const df EEst = df_sqrt(df_div(acc, df_f((float)N)));
-    ++L.attempts;
-    if (!(EEst.hi == EEst.hi)) return 4;
-    L.accept = !df_lt(df_f(1.0f), EEst);
-    // log2 EEst (EEst below 1e-30 gives the same clamped q as its exact value)
-    const df l2e = df_log2(df_max(EEst, df_f(1e-30f)), T.log2c, T.rcpc);
-    if (!L.accept) {
-        L.q11 = df_exp2(df_mul(dfc(kBeta1), l2e), T.exp2);
-        return 0;
-    }
-    df q;
-    if (EEst.hi == 0.0f) {
-        q = dfc(kQmaxInv);
-    } else {
-        // q = EEst^beta1 / qold^beta2 / gamma, clamped to [1/qmax, 1/qmin]
-        q = df_exp2(df_sub(df_mul(dfc(kBeta1), l2e), df_mul(dfc(kBeta2), L.lqold)), T.exp2);
-        q = df_max(dfc(kQmaxInv), df_min(dfc(kQminInv), df_div(q, dfc(kGamma))));
-    }
-    L.lqold = df_lt(EEst, dfc(kQoldInit)) ? dfc(kLog2QoldInit) : l2e;
-    L.elast = EEst.hi;
-    L.dtprop = df_max(df_min(L.dtmax, df_div(L.dt, q)), df_f(L.dtmin));
+    const int status = decide(L, P, T, df_sqrt(df_div(acc, df_f((float)N))));
+    if (status || !L.accept) return status;
     bool bad = false;
     for (int d = 0; d < DIM; ++d) {
         L.X[d] = Xn[d];
@@ -781,13 +802,7 @@ DFS_HD int epilogue(Lane<DIM, PHASE>& L, const DFParams& P, const Slots<KW>& k, 
         bad |= !(Xn[d].hi == Xn[d].hi) || !(Pn[d].hi == Pn[d].hi);
     }
     L.PH = PHn;
-    L.tn = L.n1;
-    L.tfr = L.f1;
-    if (L.last) return -1;
-    // within 100 ulp of t_final the FP64 solve takes t = t_final and stops
-    const df rem = df_mul(df_add(df_f((float)(P.nf - L.tn)), df_sub(d2(P.ff), L.tfr)), d2(P.h));
-    if (rem.hi < P.t_snap) return -1;
-    return bad ? 3 : 0;
+    return arrive(L, P, bad);
 }
 
 // ---- the start-up pass's hand-over -----------------------------------------------------

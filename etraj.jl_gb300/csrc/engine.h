@@ -295,7 +295,13 @@ struct DFParams {
     int threads_main, blocks_main;  // and of the main pass
     int64_t max_n;
     float* carry;           // kDfCarryWords x max_n words: electrons passed to the main pass
+    int sm_count;
+    long long few;          // electrons left below which the main pass hands them to the third
 };
+// Electrons per SM of DFParams::few: per electron the third kernel takes about three times
+// the main pass's issue slots.  12, 24, 48, 96 and 192 measured 46, 42, 41, 44 and 42 ms on 4.3e5
+// electrons with a long tail, 1.65, 1.67, 1.66, 1.64 and 1.83 ms on 1.05e5 without one.
+constexpr int kDfFewPerSm = 48;
 constexpr int kDfCarryWords = 32;        // words of one carried electron (at most 29 used)
 constexpr int kDfTablePerPeriod = 1024;  // table intervals per shortest laser period
 constexpr int kDfTableF4 = 7;            // float4 per table interval
@@ -309,8 +315,7 @@ int launch_field_table_df(const DJob& J, double T0, double h, int n_int, const D
 // Work-stealing double-float Tsit5 solve of the survivors in two passes (an
 // electron's first steps, whose error estimates need stage differences, then the
 // rest); writes out.final_state (FP64), out.status and out.steps, for
-// launch_collect_fp64.  work: three counters (start-up queue, carried electrons,
-// main-pass queue).
+// launch_collect_fp64.  work: six counters.
 int launch_integrate_df(const DFParams& P, InitSoA soa, const double* t, const int64_t* idx,
                         const unsigned long long* count, unsigned long long* work, TrajOut out,
                         cudaStream_t s);

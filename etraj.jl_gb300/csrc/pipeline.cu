@@ -240,6 +240,8 @@ void prepare_bulk(const DJob& J, double tmin, BulkParams& B) {
 // keeps busy (~4 electrons per lane).
 void prepare_df(const DJob& J, double tmin, int64_t max_n, int sm_count, DFParams& D) {
     prepare_df_params(J, tmin, max_n, D);
+    D.sm_count = sm_count;
+    D.few = (long long)sm_count * kDfFewPerSm;
     D.threads = df_threads(false);
     D.threads_main = df_threads(true);
     for (int main = 0; main < 2; ++main) {
