@@ -561,15 +561,56 @@ k_integrate_fp64_few(const __grid_constant__ DJob J, InitSoA soa, const double* 
         }
         return acc;
     };
-    // derivative of component j at the state whose components the group's lanes hold
+    // Derivative of component j at the state whose components the group's lanes hold: rhs_at
+    // (physics.cuh) with its exponentials, and its divisions, in parallel lanes.
     auto rhs_of = [&](double Fx, double Fy, double v) {
-        double w[N], du[N];
+        const DTarget& Tg = J.target;
+        const int m = lane & 7;
+        double w[N];
 #pragma unroll
         for (int i = 0; i < N; ++i) w[i] = from(v, i);
-        rhs_at<DIM, PHASE, TGT>(J, Fx, Fy, w, du);
-        double d = du[0];
+        double r2 = w[0] * w[0] + w[1] * w[1];
+        if (DIM == 3) r2 = r2 + w[2] * w[2];
+        double coef, Vphase = 0.0;
+        if (TGT == ETRAJ_TARGET_HYDROGEN_LIKE) {
+            const double q = r2 + Tg.sc, rs = DM_SQRT(q);
+            const double inv = DM_DIV(1.0, (m == 1) ? rs : q * rs);
+            coef = (-Tg.Z) * from(inv, 0);
+            if (PHASE != ETRAJ_PHASE_CTMC) Vphase = Tg.Z * from(inv, 1);
+        } else {
+            const double r = DM_SQRT(r2);
+            const double q = r * r + Tg.sc, rs = DM_SQRT(q);
+            const double ex = sae_exp(Tg, m == 0 ? Tg.b1 : m == 1 ? Tg.b2 : Tg.b3, r);
+            const double e1 = from(ex, 0), e2 = from(ex, 1), e3 = from(ex, 2);
+            const double br = (Tg.Z + (Tg.a1 * (1.0 + Tg.b1 * r)) * e1) + (Tg.a3 * (1.0 + Tg.b3 * r)) * e3;
+            const double num = ((Tg.Z + Tg.a1 * e1) + (Tg.a2 * r) * e2) + Tg.a3 * e3;
+            const double top = m == 0 ? 1.0 : m == 1 ? Tg.a2 * Tg.b2 : num;
+            const double bot = m == 0 ? q * rs : (m == 2 && DIM == 2 && PHASE == ETRAJ_PHASE_SCTS) ? q : rs;
+            const double quot = DM_DIV(top, bot);
+            coef = -(from(quot, 0) * br + from(quot, 1) * e2);
+            if (PHASE != ETRAJ_PHASE_CTMC) Vphase = from(quot, 2);
+        }
+        // a position's derivative is its momentum, a momentum's the force
+        double x = w[0], p = w[DIM];
 #pragma unroll
-        for (int i = 1; i < N; ++i) d = (j == i) ? du[i] : d;
+        for (int i = 1; i < DIM; ++i) {
+            x = (j == DIM + i) ? w[i] : x;
+            p = (j == i) ? w[DIM + i] : p;
+        }
+        double d = coef * x;
+        if (j == DIM) d = d - Fx;
+        if (j == DIM + 1) d = d - Fy;
+        if (j < DIM) d = p;
+        if (PHASE != ETRAJ_PHASE_CTMC) {
+            const double tFx = coef * w[0], tFy = coef * w[1];
+            double K = w[DIM] * w[DIM] + w[DIM + 1] * w[DIM + 1], W = w[0] * tFx + w[1] * tFy;
+            if (DIM == 3) {
+                K = K + w[5] * w[5];
+                W = W + w[2] * (coef * w[2]);
+            }
+            K = K / 2.0;
+            if (j == 2 * DIM) d = (PHASE == ETRAJ_PHASE_QTMC) ? -((Tg.Ip + K) - Vphase) : -((K - Vphase) + W);
+        }
         return d;
     };
 
