@@ -249,46 +249,55 @@ int run_batch(etraj_ctx* ctx, const etraj_job* jobs, int n, etraj_result* res, c
     return ETRAJ_OK;
 }
 
-// Copies sampled candidates back and assembles the reference's `init` columns.
+// Assembles the reference's `init` columns of candidates [g0, g0 + ng) on the device: the
+// kept ones are compacted, and k_gather_rows writes their rows into two pinned blocks in
+// turn, each copied to the caller's array while the next is written (no device memory).
+// Copying eight whole arrays back and assembling on the host took 8.0 ms for 9.6e5 3D
+// electrons, this 6.8 (the copy into fresh pages of the caller's array is 5 of them).
 int gather_rows(etraj_ctx* ctx, const HostJob& H, const Pipeline& P, int64_t g0, int64_t ng, double* init,
                 int64_t capacity, int64_t* count) {
     const DJob& J = H.J;
     cudaStream_t s = ctx->stream;
-    std::vector<uint8_t> flag((size_t)ng);
-    std::vector<double> x((size_t)ng), y((size_t)ng), kx((size_t)ng), ky((size_t)ng), kz((size_t)ng),
-        rate((size_t)ng), ph((size_t)ng);
-    std::vector<int32_t> batch((size_t)ng);
-    cudaMemcpyAsync(flag.data(), P.flag + g0, (size_t)ng, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(x.data(), P.soa.x + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(y.data(), P.soa.y + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(kx.data(), P.soa.kx + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ky.data(), P.soa.ky + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(kz.data(), P.soa.kz + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(rate.data(), P.soa.rate + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    if (P.soa.phase) cudaMemcpyAsync(ph.data(), P.soa.phase + g0, (size_t)ng * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(batch.data(), P.soa.batch + g0, (size_t)ng * 4, cudaMemcpyDeviceToHost, s);
+    launch_compact(P.flag + g0, ng, P.idx, P.block_sums, compact_blocks(ng) + 1, P.count, s);
+    unsigned long long kept = 0ull;
+    cudaMemcpyAsync(&kept, P.count, sizeof kept, cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_err(ctx, e, "sample copy-back");
-    int64_t c = 0;
-    for (int64_t i = 0; i < ng; ++i) {
-        if (!flag[(size_t)i]) continue;
-        if (c < capacity) {
-            double* r = init + c * J.rows;
-            int k = 0;
-            r[k++] = x[(size_t)i];
-            r[k++] = y[(size_t)i];
-            if (J.dim == 3) r[k++] = 0.0;
-            r[k++] = kx[(size_t)i];
-            r[k++] = ky[(size_t)i];
-            if (J.dim == 3) r[k++] = kz[(size_t)i];
-            r[k++] = H.t[(size_t)batch[(size_t)i]];
-            r[k++] = rate[(size_t)i];
-            if (J.phase != ETRAJ_PHASE_CTMC) r[k++] = ph[(size_t)i];
-        }
-        ++c;
+    if (e != cudaSuccess) return cuda_err(ctx, e, "sample count");
+    const int64_t n = std::min<int64_t>((int64_t)kept, capacity), rows = J.rows;
+    const int64_t chunk = std::min<int64_t>(n, ((int64_t)4 << 20) / (rows * 8));
+    PinnedBlock blk[2];
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    int st = ETRAJ_OK;
+    for (int b = 0; b < 2 && st == ETRAJ_OK && chunk > 0; ++b) {
+        st = get_pinned(ctx, (size_t)(chunk * rows * 8), &blk[b]);
+        done[b] = get_event(ctx);
+        if (!done[b] && st == ETRAJ_OK) st = set_err(ctx, ETRAJ_ERR_CUDA, "cudaEventCreate failed");
     }
-    *count = c;
-    return ETRAJ_OK;
+    if (st == ETRAJ_OK && chunk > 0) {
+        const int64_t chunks = (n + chunk - 1) / chunk;
+        auto len = [&](int64_t c) { return std::min(chunk, n - c * chunk); };
+        auto write = [&](int64_t c) {
+            launch_gather_rows(J, P.soa, P.t, P.idx, g0, c * chunk, len(c), (double*)blk[c & 1].p, s);
+            cudaEventRecord(done[c & 1], s);
+        };
+        write(0);
+        for (int64_t c = 0; c < chunks && e == cudaSuccess; ++c) {
+            if (c + 1 < chunks) write(c + 1);
+            e = cudaEventSynchronize(done[c & 1]);
+            if (e == cudaSuccess) std::memcpy(init + c * chunk * rows, blk[c & 1].p, (size_t)(len(c) * rows * 8));
+        }
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(s);
+            st = cuda_err(ctx, e, "sample copy-back");
+        }
+    }
+    for (int b = 0; b < 2; ++b) {
+        put_pinned(ctx, blk[b].p, blk[b].bytes);
+        if (done[b]) ctx->event_pool.push_back(done[b]);
+    }
+    if (st == ETRAJ_OK) *count = (int64_t)kept;
+    return st;
 }
 
 int sample_range(etraj_ctx* ctx, const etraj_job* job, int64_t b0, int64_t nb, double* init, int64_t capacity,

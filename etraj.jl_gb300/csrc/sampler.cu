@@ -509,6 +509,28 @@ k_compact_scatter(const uint8_t* __restrict__ flag, int64_t n, const uint32_t* _
         if (f[k]) idx[pos++] = base + k;
 }
 
+// One thread per element of the columns (ADKSampler.jl:299-303: x, y [, z], kx, ky [, kz], t,
+// rate [, phase]), so that a warp writes 256 contiguous bytes.
+__global__ void __launch_bounds__(256)
+k_gather_rows(InitSoA soa, const double* __restrict__ t, const int64_t* __restrict__ idx, int64_t g0, int64_t k0,
+              int64_t n, int rows, int dim, double* __restrict__ out) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * rows; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = e / rows, g = g0 + idx[k0 + k];
+        const int c = (int)(e - k * rows);
+        double v;
+        if (c == 0) v = soa.x[g];
+        else if (c == 1) v = soa.y[g];
+        else if (c < dim) v = 0.0;
+        else if (c == dim) v = soa.kx[g];
+        else if (c == dim + 1) v = soa.ky[g];
+        else if (c < 2 * dim) v = soa.kz[g];
+        else if (c == 2 * dim) v = t[soa.batch[g]];
+        else if (c == 2 * dim + 1) v = soa.rate[g];
+        else v = soa.phase[g];
+        out[e] = v;
+    }
+}
+
 // One thread per SPA candidate (SPASampler.jl:318-391): the same steps as the
 // CPU oracle's o_candidate_spa, in the same order.
 __global__ void __launch_bounds__(128)
@@ -653,6 +675,13 @@ int launch_sample_range(const DJob& J, int64_t b0, int64_t nb, const double* kd,
     int64_t cap = (int64_t)sm_count * 32;
     int blocks = (int)(want < cap ? (want > 0 ? want : 1) : cap);
     k_sample<<<blocks, threads, 0, s>>>(J, b0, nb, kd, kz, batches, soa, flag);
+    return 1;
+}
+
+int launch_gather_rows(const DJob& J, const InitSoA& soa, const double* t, const int64_t* idx, int64_t g0, int64_t k0,
+                       int64_t n, double* out, cudaStream_t s) {
+    const int64_t want = (n * J.rows + 255) / 256;
+    k_gather_rows<<<(unsigned)(want < 152 * 16 ? want : 152 * 16), 256, 0, s>>>(soa, t, idx, g0, k0, n, J.rows, J.dim, out);
     return 1;
 }
 
