@@ -27,7 +27,7 @@
 //    five stage times (it does not depend on the state), the components' stage and
 //    error sums and the controller's two powers run in parallel lanes: ~180 FP64
 //    instructions per attempt, for 4 electrons per warp, and a third of the latency.
-// The first kernel hands its last electrons to the second (kFewPerWarp).
+// The first kernel hands its last electrons to the second (kFewPerSm).
 // Against one lane per electron in a static grid, every evaluation in line: 1.9e5 Ar
 // trajectories 20.7 -> 17.2 ms, 1.7e5 of H2 13.2 -> 8.5 ms, 1.1e5 H 18.6 -> 8.8 ms (their
 // slowest takes 326 attempts), 1.2e3 H 14.8 -> 5.0 ms.
@@ -346,8 +346,16 @@ constexpr int state_size() {
 // use the first two turns of an attempt for their starting step.  The stage
 // derivatives are in shared memory (7 N doubles per lane).  The code is one copy of
 // the loop body, small enough for the instruction cache.
+// Blocks per SM, which sets the register budget (102 a thread for 5): with 4 the warps waited
+// for instructions and results often enough to leave the FP64 pipe 9 % idle.  5 against 4:
+// 17.2 -> 15.4 ms on 1.9e5 Ar (N = 5), 8.45 -> 8.07 on 1.7e5 H2 (N = 4); 6 spills: 17.6 and 9.0.
+// At N = 7 the stage derivatives (7 N doubles per thread) leave room for 4.
+template <int N>
+constexpr int resident_blocks() {
+    return N <= 6 ? 5 : 4;
+}
 template <int DIM, int PHASE, int TGT>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, resident_blocks<state_size<DIM, PHASE>()>())
 k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __restrict__ tsamp,
                  const int64_t* __restrict__ idx, const unsigned long long* __restrict__ count,
                  unsigned long long* __restrict__ work, TrajOut out, long long few, int one_per_warp) {
@@ -738,12 +746,11 @@ k_collect_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __rest
     }
 }
 
-// Electrons per warp of the first kernel's full grid below which the second takes over (3:
-// 7,296 electrons on 152 SMs).  The second costs 3 to 4 times the pipe time per electron:
+// Electrons per SM below which the second kernel takes over (7,296 on 152 SMs).  The second costs 3 to 4 times the pipe time per electron:
 // with all 30,011 electrons of a Ne job in it, 14.7 ms against 4.0; at 1,248 hydrogen
-// electrons with up to 347 attempts, 5.0 ms against 14.8 in the first.  1, 2, 3 and 5 measured
-// the same on jobs of 3e4 to 2e5 electrons, 10 5 % more.
-constexpr int kFewPerWarp = 3;
+// electrons with up to 347 attempts, 5.0 ms against 14.8 in the first.  16, 32, 48 and 80 measured
+// the same on jobs of 3e4 to 2e5 electrons, 160 5 % more.
+constexpr int kFewPerSm = 48;
 
 template <int DIM, int PHASE, int TGT>
 int launch_t(const DJob& J, InitSoA soa, const double* t, const int64_t* idx,
@@ -752,9 +759,9 @@ int launch_t(const DJob& J, InitSoA soa, const double* t, const int64_t* idx,
     constexpr size_t smem = (size_t)7 * state_size<DIM, PHASE>() * kThreads * sizeof(double);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(k_integrate_fp64<DIM, PHASE, TGT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int per_sm = 4, warps = kThreads / 32;
-    const int64_t grid = (int64_t)sm_count * per_sm;
-    const long long few = (long long)grid * warps * kFewPerWarp;
+    constexpr int warps = kThreads / 32;
+    const int64_t grid = (int64_t)sm_count * resident_blocks<state_size<DIM, PHASE>()>(), grid_few = (int64_t)sm_count * 4;
+    const long long few = (long long)sm_count * kFewPerSm;
     cudaMemsetAsync(work, 0, 4 * sizeof(unsigned long long), s);
     int launches = 1;
     if (max_n > few) {
@@ -764,7 +771,7 @@ int launch_t(const DJob& J, InitSoA soa, const double* t, const int64_t* idx,
         ++launches;
     }
     const int64_t want = (max_n + warps - 1) / warps;  // as many warps as electrons at most
-    k_integrate_fp64_few<DIM, PHASE, TGT><<<(unsigned)std::max<int64_t>(1, std::min(want, grid)), kThreads, 0, s>>>(
+    k_integrate_fp64_few<DIM, PHASE, TGT><<<(unsigned)std::max<int64_t>(1, std::min(want, grid_few)), kThreads, 0, s>>>(
         J, soa, t, idx, count, work, out, few, sm_count * warps);
     return launches;
 }
