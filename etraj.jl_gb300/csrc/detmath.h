@@ -255,9 +255,14 @@ DM_FN void dm_sincos_reduced(double r, int q, double* sp, double* cp) {
     double r2 = r * r;
     const fi_pair P = fi_sincos_poly(r2);
     double sr = fma(r * r2, P.s, r);
-    double hr = fi_half(r2);
-    double w = 1.0 - hr;
-    double cr = w + (((1.0 - w) - hr) + (r2 * r2) * P.c);
+    double hr = fi_half(r2), w, e;
+    if (fi_hi(hr) >= 0x3f400000u) { /* hr >= 2^-11 */
+        w = fi_one_minus(hr, &e);
+    } else {
+        w = 1.0 - hr;
+        e = (1.0 - w) - hr;
+    }
+    double cr = w + (e + (r2 * r2) * P.c);
     const double a = (q & 1) ? cr : sr, b = (q & 1) ? sr : cr;
     *sp = fi_real(fi_bits(a) ^ ((uint64_t)(uint32_t)(q & 2) << 62));
     *cp = fi_real(fi_bits(b) ^ ((uint64_t)(uint32_t)((q + 1) & 2) << 62));

@@ -231,6 +231,17 @@ FI_FN double fi_scale(double x, int k) { return fi_real(fi_bits(x) + ((uint64_t)
 FI_FN double fi_half(double x) {
     return ((fi_hi(x) & 0x7fffffffu) - 0x00200000u < 0x7fd00000u) ? fi_scale(x, -1) : 0.5 * x;
 }
+/* w = 1 - h and e = (1 - w) - h, for 2^-11 <= h < 1/2: in units of 2^-64, w the multiple of
+ * 2^11 nearest 2^64 - h (ties to even), e the exact rest */
+FI_FN double fi_one_minus(double h, double* e) {
+    const uint32_t hh = fi_hi(h);
+    const uint64_t m = ((uint64_t)((hh & 0xfffffu) | 0x100000u) << 32) | fi_lo(h);
+    const uint64_t v = 0u - (m << ((hh >> 20) - 1011u));
+    const uint64_t w = (v + 0x3ffu + ((v >> 11) & 1u)) & ~(uint64_t)0x7ff;
+    const int r = (int)(int64_t)(v - w);
+    *e = r ? fi_scale(fi_from_int(r), -64) : 0.0;
+    return fi_real((w >> 11) + ((uint64_t)1021u << 52));
+}
 FI_FN int fi_isnan(double x) { return (fi_bits(x) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull; }
 FI_FN int fi_iszero(double x) { return (fi_bits(x) << 1) == 0ull; }
 /* a < b, neither NaN */

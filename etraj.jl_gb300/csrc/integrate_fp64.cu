@@ -462,15 +462,21 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
         // ---- this turn's evaluation -----------------------------------------------------------
         if (mode == kStep) {
 #pragma unroll
-            for (int j = 0; j < N; ++j) w[j] = cA[st][0] * slot(0, j);
+            for (int j = 0; j < 2 * DIM; ++j) w[j] = cA[st][0] * slot(0, j);
 #pragma unroll 1
             for (int l = 1; l < st; ++l) {
                 const double a = cA[st][l];
 #pragma unroll
-                for (int j = 0; j < N; ++j) w[j] = fma(a, slot(l, j), w[j]);
+                for (int j = 0; j < 2 * DIM; ++j) w[j] = fma(a, slot(l, j), w[j]);
             }
 #pragma unroll
-            for (int j = 0; j < N; ++j) w[j] = fma(c.dt, w[j], u[j]);
+            for (int j = 0; j < 2 * DIM; ++j) w[j] = fma(c.dt, w[j], u[j]);
+            if (N > 2 * DIM && st == 6) {  // the phase enters no derivative: its sum is needed here only
+                double a = A71 * slot(0, N - 1);
+#pragma unroll
+                for (int l = 1; l < 6; ++l) a = fma(cA[6][l], slot(l, N - 1), a);
+                w[N - 1] = fma(c.dt, a, u[N - 1]);
+            }
             tl = (st < 5) ? fma(cC[st], c.dt, c.t) : c.t + c.dt;
         } else {
             tl = (mode == kInit) ? c.t + c.dt : c.t;

@@ -31,6 +31,7 @@ void fp_op(int op, long n, const double* x, const double* y, double* out) {
             case 22: r = fi_rint_small(x[i], &k); if ((double)k != r) r = dm_nan(); break;
             case 23: r = fi_from_int((int)x[i]); break;
             case 24: r = fi_half(x[i]); break;
+            case 28: r = fi_one_minus(x[i], &s); if (s != (1.0 - r) - x[i]) r = dm_nan(); break;
             case 25: r = fi_lt(x[i], y[i]) ? 1.0 : 0.0; break;
             default: break;
         }

@@ -89,6 +89,9 @@ def test_rounding_and_comparison(fp):
     z = np.concatenate([mantissas(rng, N), SPECIAL[::-1]])
     with np.errstate(all="ignore"):
         assert same(fp(24, x), 0.5 * x)
+    h = np.concatenate([rng.uniform(2.0 ** -11, 0.5, N), 2.0 ** -np.arange(2.0, 12.0), [np.nextafter(0.5, 0)],
+                        np.rint(rng.uniform(1, 2, N) * 2.0 ** 40) * 2.0 ** rng.integers(-51, -41, N)])
+    assert same(fp(28, h), 1.0 - h)
     ok = ~np.isnan(x) & ~np.isnan(z)
     assert np.array_equal(fp(25, x[ok], z[ok]), (x[ok] < z[ok]).astype(np.float64))
 
