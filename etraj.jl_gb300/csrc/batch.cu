@@ -126,10 +126,18 @@ int run_batch(etraj_ctx* ctx, const etraj_job* jobs, int n, etraj_result* res, c
         int launches = 0;
         rec(ctx, ctx->ev0, s);
         rec(ctx, ctx->stage_ev[0], s);
+        const DJob* jb[kMaxInstances];
+        const double* tb[kMaxInstances];
+        DBatch* ob[kMaxInstances];
+        for (int i = 0; i < n; ++i) {
+            jb[i] = &H[(size_t)i].J;
+            tb[i] = P.t + toff[i];
+            ob[i] = P.batches + toff[i];
+        }
+        launches += launch_batch_prepare_many(jb, tb, ob, n, s);
         for (int i = 0; i < n; ++i) {
             const DJob& J = H[(size_t)i].J;
             DBatch* bat = P.batches + toff[i];
-            launches += launch_batch_prepare(J, P.t + toff[i], bat, s);
             InitSoA so = P.soa;
             const int64_t c = coff[i];
             so.x += c; so.y += c; so.kx += c; so.ky += c; so.kz += c; so.rate += c; so.batch += c;
@@ -140,10 +148,12 @@ int run_batch(etraj_ctx* ctx, const etraj_job* jobs, int n, etraj_result* res, c
         rec(ctx, ctx->stage_ev[1], s);
         launches += launch_compact(P.flag, N, P.idx, P.block_sums, compact_blocks(N) + 1, P.count, s);
         rec(ctx, ctx->stage_ev[2], s);
+        std::vector<FieldTableJob> tables((size_t)n);
         for (int i = 0; i < n; ++i) {
             const BulkParams& b = B[(size_t)i];
-            launches += launch_field_table(H[(size_t)i].J, b.T0, 1.0 / b.inv_h_d, b.n_int, tab + tab_off[i], s);
+            tables[(size_t)i] = FieldTableJob{H[(size_t)i].J.laser, b.T0, 1.0 / b.inv_h_d, b.n_int, tab + tab_off[i]};
         }
+        launches += launch_field_tables(tables.data(), n, s);
         ETRAJ_TRY(tuned_bulk_launch(ctx, M, P.soa, P.t, P.idx, P.count, P.work, P.out, &launches, ctx->stage_ev + 3));
         launches += launch_collect_bulk(H[0].J, P.soa, P.t, P.idx, P.count, P.out, N, ctx->sm_count, s, d_inst, n);
         rec(ctx, ctx->stage_ev[5], s);

@@ -160,6 +160,8 @@ struct Counters {
 
 // ---- launchers (all stream-ordered; each returns the number of kernel launches) ----
 int launch_batch_prepare(const DJob& J, const double* t, DBatch* batches, cudaStream_t s);
+// The same for n atomic jobs (at most kMaxInstances) in one launch.
+int launch_batch_prepare_many(const DJob* const* jobs, const double* const* t, DBatch* const* out, int n, cudaStream_t s);
 // Samples the candidates of time samples [b0, b0+nb) (flag and SoA indexed by
 // b * n_cand + i).
 // The FP64 SPA sampler's list (the candidates its FP32 pre-pass may keep), in the
@@ -258,6 +260,14 @@ constexpr int kBulkRounds = 4;
 constexpr int kBulkCounters = 2 * kBulkRounds;  // work counter and park count per round
 constexpr int kBulkMaxIters = 1000000;  // OrdinaryDiffEq's default maxiters
 int launch_field_table(const DJob& J, double T0, double h, int n_int, float4* tab, cudaStream_t s);
+// The tables of n instances (at most kMaxInstances) in one launch.
+struct FieldTableJob {
+    DLaser laser;
+    double T0, h;
+    int n_int;
+    float4* tab;
+};
+int launch_field_tables(const FieldTableJob* jobs, int n, cudaStream_t s);
 // *out = min(*count, cap) (the autotuner's sample of the electrons)
 int launch_clamp_count(const unsigned long long* count, unsigned long long cap, unsigned long long* out,
                        cudaStream_t s);

@@ -41,6 +41,7 @@
 //
 // Roofline: FP32 issue bound, MUFU for rsqrt/exp2/log2; no tensor cores.
 
+#include <algorithm>
 #include <climits>
 
 #include "physics.cuh"
@@ -794,10 +795,18 @@ k_collect_bulk(const __grid_constant__ DJob J, InitSoA soa, const double* __rest
     }
 }
 
-__global__ void k_field_table(const __grid_constant__ DJob J, double T0, double h, int n_int,
-                              float4* __restrict__ tab) {
+template <int MAX>
+struct FieldTableJobs {
+    FieldTableJob j[MAX];
+};
+// piece k of the table of job blockIdx.y
+template <int MAX>
+__global__ void k_field_table(const __grid_constant__ FieldTableJobs<MAX> P) {
+    const FieldTableJob& J = P.j[MAX == 1 ? 0 : blockIdx.y];
+    const double T0 = J.T0, h = J.h;
+    float4* const tab = J.tab;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n_int) return;
+    if (k >= J.n_int) return;
     const double ta = T0 + (double)k * h, tb = T0 + (double)(k + 1) * h;
     double fxa, fya, dfxa, dfya, fxb, fyb, dfxb, dfyb;
     laser_F_dual(J.laser, ta, fxa, fya, dfxa, dfya);
@@ -899,7 +908,21 @@ int launch_clamp_count(const unsigned long long* count, unsigned long long cap, 
 }
 
 int launch_field_table(const DJob& J, double T0, double h, int n_int, float4* tab, cudaStream_t s) {
-    k_field_table<<<(n_int + 127) / 128, 128, 0, s>>>(J, T0, h, n_int, tab);
+    FieldTableJobs<1> P;
+    P.j[0] = FieldTableJob{J.laser, T0, h, n_int, tab};
+    k_field_table<1><<<(n_int + 127) / 128, 128, 0, s>>>(P);
+    return 1;
+}
+
+int launch_field_tables(const FieldTableJob* jobs, int n, cudaStream_t s) {
+    static_assert(sizeof(FieldTableJobs<kMaxInstances>) <= 32 * 1024, "kernel parameters hold at most 32 KB");
+    FieldTableJobs<kMaxInstances> P;
+    int most = 1;
+    for (int i = 0; i < n; ++i) {
+        P.j[i] = jobs[i];
+        most = std::max(most, jobs[i].n_int);
+    }
+    k_field_table<kMaxInstances><<<dim3((unsigned)((most + 127) / 128), (unsigned)n), 128, 0, s>>>(P);
     return 1;
 }
 
