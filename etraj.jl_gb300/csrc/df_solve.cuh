@@ -123,6 +123,7 @@ struct Slots {
         const int i = ((l - 1) * KW + 2 * c) * stride;
         return df{p[i], p[i + stride]};
     }
+    DFS_HD dfp get01(int l) const { return dfp_of(get(l, 0), get(l, 1)); }
     DFS_HD void set(int l, int c, df v) const {
         const int i = ((l - 1) * KW + 2 * c) * stride;
         p[i] = v.hi;
@@ -187,15 +188,18 @@ DFS_HD void table_piece(const DLaser& L, double T0, double h, int k, const DfTab
 // The laser table at one time: the exact c0 of each component (three floats) and
 // q(u) = u (c1 + u (c2 + u (c3 + u (c4 + ...)))) in double-float.
 struct FieldAt {
-    float c0x[3], c0y[3];
-    df qx, qy;
+    f2 c0[3];  // (x, y)
+    dfp q;
 };
 
-DFS_HD df q_of(const float* c, df u) {
-    const float t = fmaf(fmaf(fmaf(c[12], u.hi, c[11]), u.hi, c[10]), u.hi, c[9]);
-    df s = df_fma_f(t, u, df{c[7], c[8]});
-    s = df_fma(s, u, df{c[5], c[6]});
-    s = df_fma(s, u, df{c[3], c[4]});
+// (both components at once: x's coefficients at c, y's at c + 13)
+DFS_HD dfp q_of(const float* c, df u1) {
+    const dfp u = dfp_of(u1);
+    auto f = [&](int i) { return f2_of(c[i], c[13 + i]); };
+    const f2 t = dfma(dfma(dfma(f(12), u.hi, f(11)), u.hi, f(10)), u.hi, f(9));
+    dfp s = df_fma_f(t, u, dfp{f(7), f(8)});
+    s = df_fma(s, u, dfp{f(5), f(6)});
+    s = df_fma(s, u, dfp{f(3), f(4)});
     return df_mul(s, u);
 }
 
@@ -215,19 +219,16 @@ DFS_HD void field_at(const DFParams& P, int n, df f, FieldAt& F) {
         w[4 * i + 2] = v.z;
         w[4 * i + 3] = v.w;
     }
-    for (int i = 0; i < 3; ++i) {
-        F.c0x[i] = w[i];
-        F.c0y[i] = w[13 + i];
-    }
-    F.qx = q_of(w, u);
-    F.qy = q_of(w + 13, u);
+    for (int i = 0; i < 3; ++i) F.c0[i] = f2_of(w[i], w[13 + i]);
+    F.q = q_of(w, u);
 }
 
 // c0 (three floats) as a double-float
-DFS_HD df c0_df(const float* c) { return quick_two_sum(c[0], c[1] + c[2]); }
+DFS_HD dfp c0_df(const f2* c) { return quick_two_sum(c[0], c[1] + c[2]); }
+DFS_HD dfp field_df(const FieldAt& F) { return df_add(c0_df(F.c0), F.q); }
 // a - b of two exact three-float values, as a double-float
-DFS_HD df diff3(const float* a, const float* b) {
-    const df s = df_add(two_sum(a[0], -b[0]), two_sum(a[1], -b[1]));
+DFS_HD dfp diff3(const f2* a, const f2* b) {
+    const dfp s = df_add(two_sum(a[0], -b[0]), two_sum(a[1], -b[1]));
     return df_add_f(s, a[2] - b[2]);
 }
 
@@ -261,6 +262,20 @@ DFO df sae_exp(df b, df r, const float* exptab) {
     return df_exp_neg(df_neg(br), exptab);
 }
 
+// exp(-b1 r) and exp(-b3 r) at once (the same bits): the potential's long-range term b3
+// needs its exponential almost everywhere, and the other half rides along.
+DFO dfp sae_exp2(df b1, df b3, df r, const float* exptab) {
+    const dfp br = df_mul(dfp_of(b1, b3), dfp_of(r));
+    const float h0 = f2_get(br.hi, 0), h1 = f2_get(br.hi, 1);
+    const bool live0 = !(h0 > kSaeSkip) && -h0 > -87.0f, live1 = !(h1 > kSaeSkip) && -h1 > -87.0f;
+#if defined(__CUDA_ARCH__)
+    if (!__any_sync(__activemask(), live0 || live1)) return dfp{};
+#endif
+    const df z = df{0.0f, 0.0f};
+    const dfp e = df_exp_neg2(dfp_of(live0 ? df_neg(dfp_get(br, 0)) : z, live1 ? df_neg(dfp_get(br, 1)) : z), exptab);
+    return dfp_of(live0 ? dfp_get(e, 0) : z, live1 ? dfp_get(e, 1) : z);
+}
+
 // The target's terms at one state (TargetPotential / TargetForce / TrajectoryFunction,
 // HydrogenLikeAtom.jl:78-159, SAEAtom.jl:84-186): r^2 = x.x, y = (r^2 + sc)^(-1/2),
 // y^3, the force coefficient coef (F_target = coef x) and the potential term V of the
@@ -288,7 +303,8 @@ DFS_HD df phase_rate(const DFParams& P, df KE, df V, df coef_r2) {
 
 template <int DIM>
 DFS_HD df half_sq(const df* p) {
-    df s = df_add(df_sqr(p[0]), df_sqr(p[1]));
+    const dfp q = df_sqr(dfp_of(p[0], p[1]));
+    df s = df_add(dfp_get(q, 0), dfp_get(q, 1));
     if (DIM == 3) s = df_add(s, df_sqr(p[2]));
     return df{s.hi * 0.5f, s.lo * 0.5f};
 }
@@ -300,7 +316,8 @@ DFS_HD df half_sq(const df* p) {
 // and the brackets -- unless NEED_R (the start-up pass, whose differences read r).
 template <int DIM, int PHASE, int TGT, bool NEED_R = true>
 DFS_HD void target_at(const DFParams& P, const float* exptab, const df* X, const df* Pm, TAt& T, df* KT, df& kph) {
-    T.r2 = df_add(df_sqr(X[0]), df_sqr(X[1]));
+    const dfp x01 = dfp_of(X[0], X[1]), q01 = df_sqr(x01);
+    T.r2 = df_add(dfp_get(q01, 0), dfp_get(q01, 1));
     if (DIM == 3) T.r2 = df_add(T.r2, df_sqr(X[2]));
     T.y = df_rsqrt(df_add(T.r2, d2(P.sc)));
     T.y3 = df_mul(df_sqr(T.y), T.y);
@@ -312,16 +329,20 @@ DFS_HD void target_at(const DFParams& P, const float* exptab, const df* X, const
         T.coef = df_neg(df_mul(T.y3, T.br));
     } else {
         T.r = df_sqrt(T.r2);
-        T.e1 = sae_exp(d2(P.b1), T.r, exptab);
+        const dfp a = dfp_of(d2(P.a1), d2(P.a3)), b = dfp_of(d2(P.b1), d2(P.b3));
+        const dfp e = sae_exp2(d2(P.b1), d2(P.b3), T.r, exptab);
+        T.e1 = dfp_get(e, 0);
         T.e2 = sae_exp(d2(P.b2), T.r, exptab);
-        T.e3 = sae_exp(d2(P.b3), T.r, exptab);
-        T.br = df_add(df_add(d2(P.Z), df_mul(df_mul(d2(P.a1), df_add_f(df_mul(d2(P.b1), T.r), 1.0f)), T.e1)),
-                      df_mul(df_mul(d2(P.a3), df_add_f(df_mul(d2(P.b3), T.r), 1.0f)), T.e3));
-        T.num = df_add(df_add(df_add(d2(P.Z), df_mul(d2(P.a1), T.e1)), df_mul(df_mul(d2(P.a2), T.r), T.e2)),
-                       df_mul(d2(P.a3), T.e3));
+        T.e3 = dfp_get(e, 1);
+        const dfp w = df_mul(df_mul(a, df_add_f(df_mul(b, dfp_of(T.r)), splat<f2>(1.0f))), e), ae = df_mul(a, e);
+        T.br = df_add(df_add(d2(P.Z), dfp_get(w, 0)), dfp_get(w, 1));
+        T.num = df_add(df_add(df_add(d2(P.Z), dfp_get(ae, 0)), df_mul(df_mul(d2(P.a2), T.r), T.e2)), dfp_get(ae, 1));
         T.coef = df_neg(df_add(df_mul(T.y3, T.br), df_mul(df_mul(d2(P.a2b2), T.y), T.e2)));
     }
-    for (int d = 0; d < DIM; ++d) KT[d] = df_mul(T.coef, X[d]);
+    const dfp kt = df_mul(dfp_of(T.coef), x01);
+    KT[0] = dfp_get(kt, 0);
+    KT[1] = dfp_get(kt, 1);
+    if (DIM == 3) KT[2] = df_mul(T.coef, X[2]);
     if (PHASE != ETRAJ_PHASE_CTMC) {
         T.V = potential_of<DIM, PHASE, TGT>(P, T);
         kph = phase_rate<PHASE>(P, half_sq<DIM>(Pm), T.V, df_mul(T.coef, T.r2));
@@ -440,6 +461,7 @@ struct Lane {
     df dt, dth, dt2, dtprop, dtmax, lqold, q11;
     df tfr, f1, fi;           // clock fractions: accepted state, end of the attempt, evaluation
     FieldAt F5;               // laser table at the end of the attempt (stage 5), for stage 6
+    dfp Fe;                   // (the main pass: the field there, (x, y))
     df d1;                    // starting step: |f0 / sk|
     float dtmin;
     int tn, n1, ni;           // clock intervals: accepted state, end of the attempt, evaluation
@@ -491,31 +513,45 @@ DFS_HD void set_base(Lane<DIM, PHASE>& L, const FieldAt& F, const df* KT, df kph
     L.F0 = F;
     L.kph0 = kph;
     for (int d = 0; d < DIM; ++d) L.K0[d] = L.KT0[d] = KT[d];
-    L.K0[0] = df_sub(L.K0[0], df_add(c0_df(F.c0x), F.qx));
-    L.K0[1] = df_sub(L.K0[1], df_add(c0_df(F.c0y), F.qy));
+    const dfp k = df_sub(dfp_of(KT[0], KT[1]), field_df(F));
+    L.K0[0] = dfp_get(k, 0);
+    L.K0[1] = dfp_get(k, 1);
 }
 
 // dK = K - K_0 of an evaluation (target change dKT, dkph; laser table F), into slot l (1..6)
 template <int DIM, int PHASE, int KW>
 DFS_HD void set_diff(const Lane<DIM, PHASE>& L, const Slots<KW>& k, int l, const FieldAt& F, const df* dKT,
                      df dkph) {
-    const df dFx = df_add(diff3(F.c0x, L.F0.c0x), df_sub(F.qx, L.F0.qx));
-    const df dFy = df_add(diff3(F.c0y, L.F0.c0y), df_sub(F.qy, L.F0.qy));
-    k.set(l, 0, df_sub(dKT[0], dFx));
-    k.set(l, 1, df_sub(dKT[1], dFy));
+    const dfp dF = df_add(diff3(F.c0, L.F0.c0), df_sub(F.q, L.F0.q));
+    const dfp v = df_sub(dfp_of(dKT[0], dKT[1]), dF);
+    k.set(l, 0, dfp_get(v, 0));
+    k.set(l, 1, dfp_get(v, 1));
     if (DIM == 3) k.set(l, 2, dKT[2]);
     if (Lane<DIM, PHASE>::HASPH) k.set(l, DIM, dkph);
 }
 
 // The main pass keeps each stage's whole derivative instead: K_l = KT - F (the
 // momentum rows, formed as set_base forms K_0) and the phase rate, into slot l.
+// F: the field's value.
 template <int DIM, int PHASE, int KW>
-DFS_HD void set_full(const Lane<DIM, PHASE>& L, const Slots<KW>& k, int l, const FieldAt& F, const df* KT,
-                     df kph) {
-    k.set(l, 0, df_sub(KT[0], df_add(c0_df(F.c0x), F.qx)));
-    k.set(l, 1, df_sub(KT[1], df_add(c0_df(F.c0y), F.qy)));
+DFS_HD void set_full(const Lane<DIM, PHASE>& L, const Slots<KW>& k, int l, dfp F, const df* KT, df kph) {
+    const dfp v = df_sub(dfp_of(KT[0], KT[1]), F);
+    k.set(l, 0, dfp_get(v, 0));
+    k.set(l, 1, dfp_get(v, 1));
     if (DIM == 3) k.set(l, 2, KT[2]);
     if (Lane<DIM, PHASE>::HASPH) k.set(l, DIM, kph);
+}
+
+template <int DIM, int PHASE, int KW>
+DFS_HD void set_full(const Lane<DIM, PHASE>& L, const Slots<KW>& k, int l, const FieldAt& F, const df* KT, df kph) {
+    set_full(L, k, l, field_df(F), KT, kph);
+}
+
+// After stage 6 of an accepted main-pass attempt: its derivative is the new state's.
+template <int DIM, int PHASE, int KW>
+DFS_HD void base_from_full(Lane<DIM, PHASE>& L, const Slots<KW>& k) {
+    for (int d = 0; d < DIM; ++d) L.K0[d] = k.get(6, d);
+    if (Lane<DIM, PHASE>::HASPH) L.kph0 = k.get(6, DIM);
 }
 
 // sqrt(sum_j (v_j / sk_j)^2 / N)
@@ -629,19 +665,22 @@ DFS_HD int prologue(Lane<DIM, PHASE>& L, const DFParams& P) {
 
 // Sum of products c_l v_l: one TwoSum per term, the rounding errors gathered in a
 // float and normalized at the end; it may start from a double-float value.
-struct Acc {
-    float s = 0.0f, e = 0.0f;
-    DFS_HD Acc() {}
-    DFS_HD explicit Acc(df v) : s(v.hi), e(v.lo) {}
-    DFS_HD void add(df c, df v) {
-        const df p = two_prod(c.hi, v.hi);
-        const float pe = fmaf(c.hi, v.lo, fmaf(c.lo, v.hi, p.lo));
-        const df t = two_sum(s, p.hi);
+template <class T>
+struct AccT {
+    T s = {}, e = {};
+    DFS_HD AccT() {}
+    DFS_HD explicit AccT(dft<T> v) : s(v.hi), e(v.lo) {}
+    DFS_HD void add(dft<T> c, dft<T> v) {
+        const dft<T> p = two_prod(c.hi, v.hi);
+        const T pe = dfma(c.hi, v.lo, dfma(c.lo, v.hi, p.lo));
+        const dft<T> t = two_sum(s, p.hi);
         s = t.hi;
         e += t.lo + pe;
     }
-    DFS_HD df get() const { return two_sum(s, e); }
+    DFS_HD dft<T> get() const { return two_sum(s, e); }
 };
+using Acc = AccT<float>;
+using AccP = AccT<f2>;  // of the x and y components
 
 // The increments and clock of stage st (1..6; 6 is the new state):
 // dP = dt ((sum_l A_l) K_0 + sum_l A_l dK_l) and
@@ -652,7 +691,23 @@ struct Acc {
 template <bool FULL, int DIM, int PHASE, int KW>
 DFS_HD void stage_in(Lane<DIM, PHASE>& L, const Slots<KW>& k, int st) {
     const df adt = df_mul(DFS_T RA[st], L.dt);
-    for (int d = 0; d < DIM; ++d) {
+    {
+        const dfp K0 = dfp_of(L.K0[0], L.K0[1]);
+        AccP sa(df_mul(dfp_of(FULL ? DFS_T A[st][0] : DFS_T RA[st]), K0)),
+            saa(df_mul(dfp_of(FULL ? DFS_T AA[st][0] : DFS_T RAA[st]), K0));
+        for (int l = 1; l < st; ++l) {
+            const dfp kl = k.get01(l);
+            sa.add(dfp_of(DFS_T A[st][l]), kl);
+            if (l + 1 < st) saa.add(dfp_of(DFS_T AA[st][l]), kl);  // (A A)[st][st-1] = 0
+        }
+        const dfp dp = df_mul(dfp_of(L.dt), sa.get());
+        const dfp dx = df_fma(dfp_of(adt), dfp_of(L.Pv[0], L.Pv[1]), df_mul(dfp_of(L.dt2), saa.get()));
+        for (int d = 0; d < 2; ++d) {
+            L.dP[d] = dfp_get(dp, d);
+            L.dX[d] = dfp_get(dx, d);
+        }
+    }
+    for (int d = 2; d < DIM; ++d) {
         Acc sa(df_mul(FULL ? DFS_T A[st][0] : DFS_T RA[st], L.K0[d])),
             saa(df_mul(FULL ? DFS_T AA[st][0] : DFS_T RAA[st], L.K0[d]));
         for (int l = 1; l < st; ++l) {
@@ -690,7 +745,13 @@ DFS_HD void target_eval(const DFParams& P, const float* exptab, const Lane<DIM, 
     if (DIFF && diff) ok = target_diff<DIM, PHASE, TGT>(P, exptab, L.X, L.Pv, B, L.dX, L.dP, dKT, dkph);
     if (direct || !ok) {
         df Xl[DIM], Pl[DIM];
-        for (int d = 0; d < DIM; ++d) {
+        const dfp x = df_add(dfp_of(L.X[0], L.X[1]), dfp_of(L.dX[0], L.dX[1]));
+        const dfp p = df_add(dfp_of(L.Pv[0], L.Pv[1]), dfp_of(L.dP[0], L.dP[1]));
+        for (int d = 0; d < 2; ++d) {
+            Xl[d] = dfp_get(x, d);
+            Pl[d] = dfp_get(p, d);
+        }
+        for (int d = 2; d < DIM; ++d) {
             Xl[d] = df_add(L.X[d], L.dX[d]);
             Pl[d] = df_add(L.Pv[d], L.dP[d]);
         }
@@ -751,20 +812,56 @@ template <bool FULL, int DIM, int PHASE, int KW>
 DFS_HD int epilogue(Lane<DIM, PHASE>& L, const DFParams& P, const Slots<KW>& k, const Tabs& T) {
     constexpr bool HASPH = Lane<DIM, PHASE>::HASPH;
     constexpr int N = Lane<DIM, PHASE>::N;
-    df dPH = df{0.0f, 0.0f};
-    if (HASPH) {
-        Acc a(df_mul(FULL ? DFS_T A[6][0] : DFS_T RA[6], L.kph0));
+    df dPH = df{0.0f, 0.0f}, ePH = df{0.0f, 0.0f};
+    if (HASPH) {  // the phase's stage sum and error sum at once
+        const dfp a0 = df_mul(dfp_of(FULL ? DFS_T A[6][0] : DFS_T RA[6], DFS_T BT[0]), dfp_of(L.kph0));
+        AccP a(FULL ? a0 : dfp_of(dfp_get(a0, 0), ePH));
 #pragma unroll
-        for (int l = 1; l < 6; ++l) a.add(DFS_T A[6][l], k.get(l, DIM));
-        dPH = df_mul(L.dt, a.get());
+        for (int l = 1; l < 6; ++l) a.add(dfp_of(DFS_T A[6][l], DFS_T BT[l]), dfp_of(k.get(l, DIM)));
+        Acc ef(df{f2_get(a.s, 1), f2_get(a.e, 1)});
+        ef.add(DFS_T BT[6], k.get(6, DIM));
+        dPH = df_mul(L.dt, two_sum(f2_get(a.s, 0), f2_get(a.e, 0)));
+        ePH = df_mul(L.dt, ef.get());
     }
     const df PHn = df_add(L.PH, dPH);
     // RMS of the error estimate over the scales abstol + rtol max(|u_prev|, |u_new|);
     // the weights of K_0 (sum bt, sum bt A) are 0 on differences
     df acc = df{0.0f, 0.0f};
     df Xn[DIM], Pn[DIM];
+    {
+        AccP ex, ep;
+        if (FULL) {
+            const dfp K0 = dfp_of(L.K0[0], L.K0[1]);
+            ex = AccP(df_mul(dfp_of(DFS_T BTA[0]), K0));
+            ep = AccP(df_mul(dfp_of(DFS_T BT[0]), K0));
+        }
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) {
+        for (int l = 1; l < 7; ++l) {
+            const dfp kl = k.get01(l);
+            if (l < 6) ex.add(dfp_of(DFS_T BTA[l]), kl);  // (bt A)[6] = 0
+            ep.add(dfp_of(DFS_T BT[l]), kl);
+        }
+        const dfp xn = df_add(dfp_of(L.X[0], L.X[1]), dfp_of(L.dX[0], L.dX[1]));
+        const dfp pn = df_add(dfp_of(L.Pv[0], L.Pv[1]), dfp_of(L.dP[0], L.dP[1]));
+        const dfp vx = df_mul(dfp_of(L.dt2), ex.get()), vp = df_mul(dfp_of(L.dt), ep.get());
+        df mx[2], mp[2];
+        for (int d = 0; d < 2; ++d) {
+            Xn[d] = dfp_get(xn, d);
+            Pn[d] = dfp_get(pn, d);
+            mx[d] = df_max(df_abs(L.X[d]), df_abs(Xn[d]));
+            mp[d] = df_max(df_abs(L.Pv[d]), df_abs(Pn[d]));
+        }
+        const dfp rtol = dfp_of(d2(P.rtol)), atol = dfp_of(dfc(kAbstol));
+        const dfp scx = df_fma(dfp_of(mx[0], mx[1]), rtol, atol), scp = df_fma(dfp_of(mp[0], mp[1]), rtol, atol);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const df rx = df_div(dfp_get(vx, d), dfp_get(scx, d));
+            const df rp = df_div(dfp_get(vp, d), dfp_get(scp, d));
+            acc = df_fma(rx, rx, df_fma(rp, rp, acc));
+        }
+    }
+#pragma unroll
+    for (int d = 2; d < DIM; ++d) {
         Acc ex, ep;
         if (FULL) {
             ex = Acc(df_mul(DFS_T BTA[0], L.K0[d]));
@@ -785,12 +882,8 @@ DFS_HD int epilogue(Lane<DIM, PHASE>& L, const DFParams& P, const Slots<KW>& k, 
         acc = df_fma(rx, rx, df_fma(rp, rp, acc));
     }
     if (HASPH) {
-        Acc ef;
-        if (FULL) ef = Acc(df_mul(DFS_T BT[0], L.kph0));
-#pragma unroll
-        for (int l = 1; l < 7; ++l) ef.add(DFS_T BT[l], k.get(l, DIM));
         const df scf = df_fma(df_max(df_abs(L.PH), df_abs(PHn)), d2(P.rtol), dfc(kAbstol));
-        const df rf = df_div(df_mul(L.dt, ef.get()), scf);
+        const df rf = df_div(ePH, scf);
         acc = df_fma(rf, rf, acc);
     }
     const int status = decide(L, P, T, df_sqrt(df_div(acc, df_f((float)N))));

@@ -33,27 +33,101 @@
 
 namespace etraj {
 
-struct df {
-    float hi, lo;
+// Two floats in a 64-bit register, one operation on both: GB300 adds such a pair, or fuses
+// its product and sum, in one instruction that rounds each half as the scalar one does.
+// The pipe takes two cycles for it (2.0 measured), so it saves issue slots and code, not
+// pipe time.  With the x and y components in pairs wherever both go through the same
+// operations the integrator takes 67.7 -> 62.0 ms on 4.0e6 argon electrons.
+struct f2 {
+    unsigned long long v;
 };
+DFI f2 f2_of(float a, float b) {
+    f2 r;
+#if defined(__CUDA_ARCH__)
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+#else
+    std::memcpy(&r.v, &a, 4);
+    std::memcpy((char*)&r.v + 4, &b, 4);
+#endif
+    return r;
+}
+DFI float f2_get(f2 x, int i) {
+    float a, b;
+#if defined(__CUDA_ARCH__)
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+#else
+    std::memcpy(&a, &x.v, 4);
+    std::memcpy(&b, (const char*)&x.v + 4, 4);
+#endif
+    return i ? b : a;
+}
+#if defined(__CUDA_ARCH__)
+#define ETRAJ_F2_OP(name, ptx, op)                                           \
+    DFI f2 name(f2 x, f2 y) {                                                \
+        f2 r;                                                                \
+        asm(ptx ".rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));   \
+        return r;                                                            \
+    }
+#else
+#define ETRAJ_F2_OP(name, ptx, op) \
+    DFI f2 name(f2 x, f2 y) { return f2_of(f2_get(x, 0) op f2_get(y, 0), f2_get(x, 1) op f2_get(y, 1)); }
+#endif
+ETRAJ_F2_OP(operator+, "add", +)
+ETRAJ_F2_OP(operator-, "sub", -)
+#undef ETRAJ_F2_OP
+DFI f2 operator-(f2 x) { return f2_of(-f2_get(x, 0), -f2_get(x, 1)); }
+DFI f2& operator+=(f2& x, f2 y) { return x = x + y; }
+template <class T>
+DFI T splat(float a);
+template <>
+DFI float splat<float>(float a) { return a; }
+template <>
+DFI f2 splat<f2>(float a) { return f2_of(a, a); }
+// Products one half at a time: ptxas (13.0) fuses a packed product, though written with
+// .rn, into the packed sum it feeds, which rounds once where the source says twice.
+DFI f2 operator*(f2 x, f2 y) { return f2_of(f2_get(x, 0) * f2_get(y, 0), f2_get(x, 1) * f2_get(y, 1)); }
+DFI float dfma(float a, float b, float c) { return fmaf(a, b, c); }
+DFI f2 dfma(f2 a, f2 b, f2 c) {
+#if defined(__CUDA_ARCH__)
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+#else
+    return f2_of(fmaf(f2_get(a, 0), f2_get(b, 0), f2_get(c, 0)), fmaf(f2_get(a, 1), f2_get(b, 1), f2_get(c, 1)));
+#endif
+}
+
+// a double-float (T = float), or a pair of them (T = f2)
+template <class T>
+struct dft {
+    T hi, lo;
+};
+using df = dft<float>;
+using dfp = dft<f2>;
 
 DFI df df_f(float h) { return df{h, 0.0f}; }
+DFI dfp dfp_of(df a, df b) { return dfp{f2_of(a.hi, b.hi), f2_of(a.lo, b.lo)}; }
+DFI dfp dfp_of(df a) { return dfp_of(a, a); }
+DFI df dfp_get(dfp a, int i) { return df{f2_get(a.hi, i), f2_get(a.lo, i)}; }
 
 // s + e = a + b exactly (Knuth's TwoSum)
-DFI df two_sum(float a, float b) {
-    const float s = a + b;
-    const float bb = s - a;
-    return df{s, (a - (s - bb)) + (b - bb)};
+template <class T>
+DFI dft<T> two_sum(T a, T b) {
+    const T s = a + b;
+    const T bb = s - a;
+    return dft<T>{s, (a - (s - bb)) + (b - bb)};
 }
 // s + e = a + b exactly, given |a| >= |b| or a == 0 (Dekker's Fast2Sum)
-DFI df quick_two_sum(float a, float b) {
-    const float s = a + b;
-    return df{s, b - (s - a)};
+template <class T>
+DFI dft<T> quick_two_sum(T a, T b) {
+    const T s = a + b;
+    return dft<T>{s, b - (s - a)};
 }
 // p + e = a * b exactly
-DFI df two_prod(float a, float b) {
-    const float p = a * b;
-    return df{p, fmaf(a, b, -p)};
+template <class T>
+DFI dft<T> two_prod(T a, T b) {
+    const T p = a * b;
+    return dft<T>{p, dfma(a, b, -p)};
 }
 
 // nearest double-float of an FP64 value (FP64 operations: use at load/store only)
@@ -63,23 +137,28 @@ DFI df df_from_double(double x) {
 }
 DFI double df_to_double(df a) { return (double)a.hi + (double)a.lo; }
 
-DFI df df_neg(df a) { return df{-a.hi, -a.lo}; }
+template <class T>
+DFI dft<T> df_neg(dft<T> a) { return dft<T>{-a.hi, -a.lo}; }
 DFI df df_abs(df a) { return a.hi < 0.0f ? df{-a.hi, -a.lo} : a; }
 
-DFI df df_add(df a, df b) {
-    df s = two_sum(a.hi, b.hi);
+template <class T>
+DFI dft<T> df_add(dft<T> a, dft<T> b) {
+    dft<T> s = two_sum(a.hi, b.hi);
     s.lo += a.lo + b.lo;
     return quick_two_sum(s.hi, s.lo);
 }
-DFI df df_sub(df a, df b) { return df_add(a, df_neg(b)); }
-DFI df df_add_f(df a, float b) {
-    df s = two_sum(a.hi, b);
+template <class T>
+DFI dft<T> df_sub(dft<T> a, dft<T> b) { return df_add(a, df_neg(b)); }
+template <class T>
+DFI dft<T> df_add_f(dft<T> a, T b) {
+    dft<T> s = two_sum(a.hi, b);
     s.lo += a.lo;
     return quick_two_sum(s.hi, s.lo);
 }
-DFI df df_mul(df a, df b) {
-    df p = two_prod(a.hi, b.hi);
-    p.lo = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, p.lo));
+template <class T>
+DFI dft<T> df_mul(dft<T> a, dft<T> b) {
+    dft<T> p = two_prod(a.hi, b.hi);
+    p.lo = dfma(a.hi, b.lo, dfma(a.lo, b.hi, p.lo));
     return quick_two_sum(p.hi, p.lo);
 }
 DFI df df_mul_f(df a, float b) {
@@ -87,24 +166,27 @@ DFI df df_mul_f(df a, float b) {
     p.lo = fmaf(a.lo, b, p.lo);
     return quick_two_sum(p.hi, p.lo);
 }
-DFI df df_sqr(df a) {
-    df p = two_prod(a.hi, a.hi);
-    p.lo = fmaf(a.hi + a.hi, a.lo, p.lo);
+template <class T>
+DFI dft<T> df_sqr(dft<T> a) {
+    dft<T> p = two_prod(a.hi, a.hi);
+    p.lo = dfma(a.hi + a.hi, a.lo, p.lo);
     return quick_two_sum(p.hi, p.lo);
 }
 // a * b + c with one renormalization
-DFI df df_fma(df a, df b, df c) {
-    df p = two_prod(a.hi, b.hi);
-    const float e = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, p.lo));
-    df s = two_sum(p.hi, c.hi);
+template <class T>
+DFI dft<T> df_fma(dft<T> a, dft<T> b, dft<T> c) {
+    dft<T> p = two_prod(a.hi, b.hi);
+    const T e = dfma(a.hi, b.lo, dfma(a.lo, b.hi, p.lo));
+    dft<T> s = two_sum(p.hi, c.hi);
     s.lo += e + c.lo;
     return quick_two_sum(s.hi, s.lo);
 }
 // a * b + c for a float a
-DFI df df_fma_f(float a, df b, df c) {
-    df p = two_prod(a, b.hi);
-    const float e = fmaf(a, b.lo, p.lo);
-    df s = two_sum(p.hi, c.hi);
+template <class T>
+DFI dft<T> df_fma_f(T a, dft<T> b, dft<T> c) {
+    dft<T> p = two_prod(a, b.hi);
+    const T e = dfma(a, b.lo, p.lo);
+    dft<T> s = two_sum(p.hi, c.hi);
     s.lo += e + c.lo;
     return quick_two_sum(s.hi, s.lo);
 }
@@ -422,36 +504,53 @@ constexpr float kRcpcTab[2 * kLogTabN] = {ETRAJ_DF_RCPC_TABLE};
 
 // exp(r) - 1 for |r| <= ~1.4e-3: r + r^2/2 in double-float, r^3/6 + r^4/24 in FP32
 // (below 4.2e-10 and 1.4e-13), the truncation r^5/120 < 4e-17
-DFI df df_expm1_small(df r) {
-    df r2 = df_sqr(r);
-    r2.hi *= 0.5f;
-    r2.lo *= 0.5f;
-    const float tail = (r.hi * r.hi) * (r.hi * fmaf(r.hi, 1.0f / 24.0f, 1.0f / 6.0f));
+template <class T>
+DFI dft<T> df_expm1_small(dft<T> r) {
+    dft<T> r2 = df_sqr(r);
+    r2.hi = r2.hi * splat<T>(0.5f);
+    r2.lo = r2.lo * splat<T>(0.5f);
+    const T tail = (r.hi * r.hi) * (r.hi * dfma(r.hi, splat<T>(1.0f / 24.0f), splat<T>(1.0f / 6.0f)));
     return df_add_f(df_add(r, r2), tail);
 }
 // 2^(j/256) (1 + p) 2^m for -126 <= m <= 127, n = 256 m + j
-DFI df df_exp_assemble(int n, df p, const float* tab) {
+DFI df df_exp_entry(int n, const float* tab, float& sc) {
     const int j = n & (kExpTabN - 1);
     const int m = n >> 8;  // floor(n / 256)
-    const df T = df{tab[2 * j], tab[2 * j + 1]};
-    const df e = df_fma(T, p, T);
     const uint32_t bits = (uint32_t)(m + 127) << 23;
-    float sc;
     std::memcpy(&sc, &bits, sizeof sc);
+    return df{tab[2 * j], tab[2 * j + 1]};
+}
+DFI df df_exp_assemble(int n, df p, const float* tab) {
+    float sc;
+    const df T = df_exp_entry(n, tab, sc);
+    const df e = df_fma(T, p, T);
     return df{e.hi * sc, e.lo * sc};
 }
 
+// r = x - n ln2/256: x.hi - n L1 is exact (n L1 has <= 24 bits and is within a
+// factor of 2 of x.hi, or r is tiny)
+template <class T>
+DFI dft<T> df_exp_reduce(dft<T> x, T n) {
+    dft<T> r = two_sum(dfma(-n, splat<T>(kExpL1), x.hi), x.lo);
+    r = df_add(r, two_prod(-n, splat<T>(kExpL2)));
+    r.lo = dfma(-n, splat<T>(kExpL3), r.lo);
+    return quick_two_sum(r.hi, r.lo);
+}
 // exp(x) for x <= 0 (results below 2^-126 are returned as 0); tab: ETRAJ_DF_EXP2_TABLE
 DFI df df_exp_neg(df x, const float* tab) {
     if (!(x.hi > -87.0f)) return df{0.0f, 0.0f};
     const float n = rintf(x.hi * kExpInvL);
-    // r = x - n ln2/256: x.hi - n L1 is exact (n L1 has <= 24 bits and is within a
-    // factor of 2 of x.hi, or r is tiny)
-    df r = two_sum(fmaf(-n, kExpL1, x.hi), x.lo);
-    r = df_add(r, two_prod(-n, kExpL2));
-    r.lo = fmaf(-n, kExpL3, r.lo);
-    r = quick_two_sum(r.hi, r.lo);
-    return df_exp_assemble((int)n, df_expm1_small(r), tab);
+    return df_exp_assemble((int)n, df_expm1_small(df_exp_reduce(x, n)), tab);
+}
+// the same for a pair, both above -87
+DFI dfp df_exp_neg2(dfp x, const float* tab) {
+    const float n0 = rintf(f2_get(x.hi, 0) * kExpInvL), n1 = rintf(f2_get(x.hi, 1) * kExpInvL);
+    const dfp p = df_expm1_small(df_exp_reduce(x, f2_of(n0, n1)));
+    float s0, s1;
+    const df t0 = df_exp_entry((int)n0, tab, s0), t1 = df_exp_entry((int)n1, tab, s1);
+    const dfp T = dfp_of(t0, t1), e = df_fma(T, p, T);
+    const f2 sc = f2_of(s0, s1);
+    return dfp{e.hi * sc, e.lo * sc};
 }
 
 // 2^x for -126 <= x < 127: x = n/256 + r (x.hi - n/256 is exact), |r| <= 1/512,

@@ -37,8 +37,13 @@
 // double-float pairs, c4..c7 as floats), 112 B per piece read through the L1
 // cache.  Time is a clock of an integer piece index and a double-float fraction.
 //
-// Roofline: FP32 issue bound (a double-float add is ~11 FP32 instructions, a
-// product ~7); no tensor cores (not a contraction).  Compiled with
+// What bounds it: FP32 instructions (a double-float add is 11, a product 7); no tensor
+// cores (not a contraction).  The x and y components share an instruction (dfloat.h, f2),
+// and so do the two longer-ranged exponentials of an SAE potential: in the main pass on
+// 4e5 argon electrons 63 % of the issue slots and 54 % of the FP32 pipe are then in use,
+// and the rest goes to the latency of dependent instructions with four warps per scheduler,
+// which is what 128 registers a thread leave (five warps at 96 registers spill: 67.7 ms
+// against 64.3 on 4.0e6 argon electrons).  Compiled with
 // --fmad=false: every fused multiply-add is an explicit fmaf(), as the
 // error-free transformations need.
 
@@ -214,8 +219,14 @@ k_integrate_df(const __grid_constant__ DFParams P, InitSoA soa, const double* __
         if (mode == kStep || mode == kInit1 || mode == kBase) {
             const bool step6 = (mode == kStep && st == 6);
             dfs::FieldAt F;
-            if (step6) F = L.F5;  // stage 6 is at stage 5's time
-            else dfs::field_at(P, L.ni, L.fi, F);
+            dfp Fv = {};  // the field's value (the main pass needs no more)
+            if (step6) {  // stage 6 is at stage 5's time
+                if (MAIN) Fv = L.Fe;
+                else F = L.F5;
+            } else {
+                dfs::field_at(P, L.ni, L.fi, F);
+                if (MAIN) Fv = dfs::field_df(F);
+            }
             const bool diff = !MAIN && mode != kBase;
             dfs::TAt Tl;
             df KT[DIM], dKT[DIM], dkph, kph;
@@ -225,20 +236,25 @@ k_integrate_df(const __grid_constant__ DFParams P, InitSoA soa, const double* __
                 dfs::set_base(L, F, KT, kph);
                 mode = (!MAIN && dfs::init_first(L, P)) ? kInit1 : kWait;
             } else {
-                if (MAIN) dfs::set_full(L, ks, st, F, KT, kph);
+                if (MAIN) dfs::set_full(L, ks, st, Fv, KT, kph);
                 else dfs::set_diff(L, ks, (mode == kInit1) ? 1 : st, F, dKT, dkph);
                 if (mode == kInit1) {
                     dfs::init_second(L, P, ks, T);
                     mode = kWait;
                 } else if (st == 5) {
-                    L.F5 = F;
+                    if (MAIN) L.Fe = Fv;
+                    else L.F5 = F;
                 } else if (step6) {
                     const int status = dfs::epilogue<MAIN>(L, P, ks, T);
                     if (status) {
                         finish(status < 0 ? 0 : status);
                     } else if (L.accept) {
-                        if (!MAIN) B = Tl;
-                        dfs::set_base(L, L.F5, KT, kph);
+                        if (MAIN) {
+                            dfs::base_from_full(L, ks);
+                        } else {
+                            B = Tl;
+                            dfs::set_base(L, L.F5, KT, kph);
+                        }
                     }
                 }
             }
@@ -254,7 +270,7 @@ k_integrate_df(const __grid_constant__ DFParams P, InitSoA soa, const double* __
 // the start of the attempt, the target in all of them.  Every double-float operation is
 // the main pass's, so the bits are too (a term with a zero weight changes no sum).
 // Measured: 87 -> 42 ms for 4.3e5 hydrogen electrons in a two-colour field (the slowest takes
-// 5441 attempts, 7.6 us each here), 2.02 -> 1.62 ms for 1.05e5 of a linear pulse; with the
+// 5441 attempts, 7.3 us each here), 2.02 -> 1.62 ms for 1.05e5 of a linear pulse; with the
 // hand-over's code in the main pass, 67.0 -> 67.7 ms on 4.0e6 argon electrons.  Handing over
 // by a warp's own count of lanes (4, 8, 12, 16) left the linear job at 1.8 to 2.0 ms.
 constexpr int kDfThreadsFew = 128;
@@ -320,7 +336,8 @@ k_integrate_df_few(const __grid_constant__ DFParams P, unsigned long long* __res
                 if (d == i) S = pos ? L.X[i] : L.Pv[i];
             dfs::FieldAt F;
             dfs::field_at(P, L.ni, L.fi, F);
-            K0 = derivative(df_add(S, df_f(0.0f)), df_add(dfs::c0_df(F.c0x), F.qx), df_add(dfs::c0_df(F.c0y), F.qy));
+            const dfp f0 = dfs::field_df(F);
+            K0 = derivative(df_add(S, df_f(0.0f)), dfp_get(f0, 0), dfp_get(f0, 1));
             active = true;
         }
         int status = dfs::prologue(L, P);
@@ -331,7 +348,8 @@ k_integrate_df_few(const __grid_constant__ DFParams P, unsigned long long* __res
             if (m < 4) dfs::clk_adv(L.tn, L.tfr, df_mul(dfs::DFS_T C[m + 1], L.dth), ni, fi);
             dfs::FieldAt F;
             dfs::field_at(P, ni, fi, F);
-            const df Fx = df_add(dfs::c0_df(F.c0x), F.qx), Fy = df_add(dfs::c0_df(F.c0y), F.qy);
+            const dfp Fd = dfs::field_df(F);
+            const df Fx = dfp_get(Fd, 0), Fy = dfp_get(Fd, 1);
             const df Pd = from(S, d), step = pick(L.dt2, L.dt);
             df K[7], V = S;
             K[0] = K0;
