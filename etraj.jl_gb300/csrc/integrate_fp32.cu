@@ -219,7 +219,10 @@ __device__ __forceinline__ float small_int_to_float(int k) {
 // five table reads of an attempt go first, in flight together, instead of each being
 // waited for in its stage: 2.34 -> 1.73 us an attempt of a lone electron in a 40-cycle
 // pulse, 38.0 -> 37.1 ms for a batch of 16 instances.  With the table in shared memory
-// the early reads only hold registers (5.23 -> 5.39 ms on 4.0e6 electrons).
+// the early reads only hold registers (5.23 -> 5.39 ms on 4.0e6 electrons).  A single job
+// uses them in the rounds after the first, which carry its slowest electrons: in the first
+// the registers (125 instead of 96 for hydrogen) keep other jobs' blocks off the SM
+// (512 requests on 8 slots: p50 1.2 to 1.5 s instead of 0.5 to 0.8).
 // OCC: resident 256-thread blocks per SM the build is held to (2: <= 128
 // registers per thread, 16 warps per SM; 3: <= 85 registers, 24 warps).
 template <int DIM, int PHASE, int TGT, bool MULTI, bool EARLY, int OCC>
@@ -825,10 +828,11 @@ int launch_bulk_t(const BulkParams& P, InitSoA soa, const double* t, const int64
                   const unsigned long long* count, unsigned long long* queue, TrajOut out, int sm_count,
                   cudaStream_t s) {
     const size_t smem = (!MULTI && P.table_in_smem) ? (size_t)P.n_int * 2 * sizeof(float4) : 0;
-    auto kern = (P.occ == 3) ? (smem ? k_integrate_bulk<DIM, PHASE, TGT, MULTI, MULTI, 3>
-                                    : k_integrate_bulk<DIM, PHASE, TGT, MULTI, true, 3>)
-                             : (smem ? k_integrate_bulk<DIM, PHASE, TGT, MULTI, MULTI, 2>
-                                     : k_integrate_bulk<DIM, PHASE, TGT, MULTI, true, 2>);
+    auto kern = (P.occ == 3) ? k_integrate_bulk<DIM, PHASE, TGT, MULTI, MULTI, 3>
+                             : k_integrate_bulk<DIM, PHASE, TGT, MULTI, MULTI, 2>;
+    auto late = smem ? kern  // of the rounds after the first
+                     : (P.occ == 3) ? k_integrate_bulk<DIM, PHASE, TGT, MULTI, true, 3>
+                                    : k_integrate_bulk<DIM, PHASE, TGT, MULTI, true, 2>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // persistent grid, but no more blocks than the job can keep busy (at least ~4
     // electrons per lane): a block holds its SM's registers until its last warp
@@ -865,7 +869,8 @@ int launch_bulk_t(const BulkParams& P, InitSoA soa, const double* t, const int64
         Q.park_in_count = (r > 0) ? queue + 2 * (r - 1) + 1 : nullptr;
         Q.park_out = (P.park_buf && r + 1 < rounds) ? P.park_buf + (size_t)(r & 1) * half : nullptr;
         Q.park_out_count = queue + 2 * r + 1;
-        kern<<<(r == 0) ? blocks : (int)cap, P.threads, smem, s>>>(Q, soa, t, idx, count, queue + 2 * r, out);
+        (r == 0 ? kern : late)<<<(r == 0) ? blocks : (int)cap, P.threads, smem, s>>>(Q, soa, t, idx, count, queue + 2 * r,
+                                                                                   out);
     }
     return rounds;
 }
