@@ -28,9 +28,9 @@
 //    error sums and the controller's two powers run in parallel lanes: ~180 FP64
 //    instructions per attempt, for 4 electrons per warp, and a third of the latency.
 // The first kernel hands its last electrons to the second (kFewPerSm).
-// Against one lane per electron in a static grid, every evaluation in line: 1.9e5 Ar
-// trajectories 20.7 -> 17.2 ms, 1.7e5 of H2 13.2 -> 8.5 ms, 1.1e5 H 18.6 -> 8.8 ms (their
-// slowest takes 326 attempts), 1.2e3 H 14.8 -> 5.0 ms.
+// Against one lane per electron in a static grid, with the same arithmetic: 1.9e5 Ar
+// trajectories 20.7 -> 15.0 ms, 1.7e5 of H2 13.2 -> 7.9 ms, 1.1e5 H 18.6 -> 8.4 ms (their
+// slowest takes 326 attempts), 1.2e3 H 14.8 -> 4.7 ms.
 
 #include <algorithm>
 
