@@ -29,7 +29,7 @@
 //    instructions per attempt, for 4 electrons per warp, and a third of the latency.
 // The first kernel hands its last electrons to the second (kFewPerSm).
 // Against one lane per electron in a static grid, with the same arithmetic: 1.9e5 Ar
-// trajectories 20.7 -> 15.0 ms, 1.7e5 of H2 13.2 -> 7.9 ms, 1.1e5 H 18.6 -> 8.4 ms (their
+// trajectories 20.7 -> 14.3 ms, 1.7e5 of H2 13.2 -> 7.6 ms, 1.1e5 H 18.6 -> 8.4 ms (their
 // slowest takes 326 attempts), 1.2e3 H 14.8 -> 4.7 ms.
 
 #include <algorithm>
@@ -344,10 +344,14 @@ constexpr int state_size() {
 // One electron per lane.  A warp goes through the stages in step: stage st = 1..6 of
 // every stepping lane, one evaluation of the right-hand side per turn; new electrons
 // use the first two turns of an attempt for their starting step.  The stage
-// derivatives are in shared memory (7 N doubles per lane).  The code is one copy of
-// the loop body, small enough for the instruction cache.
+// derivatives are in shared memory (7 N doubles per lane).
+// The loop body is larger than the instruction cache: with four and five warps per
+// sub-partition a third of the time between a warp's instructions went to fetching.  So
+// above two a block's warps go through the turns in step, a barrier at each, and share what
+// they fetch: 15.0 -> 14.3 ms on 1.9e5 Ar, 7.9 -> 7.6 on 1.7e5 H2.  With two (3.0e4 Ne) the
+// barrier costs more than it saves (a call 4.0 -> 4.2 ms).
 // Blocks per SM, which sets the register budget (102 a thread for 5): with 4 the warps waited
-// for instructions and results often enough to leave the FP64 pipe 9 % idle.  5 against 4:
+// for instructions and results more of the time.  5 against 4:
 // 17.2 -> 15.4 ms on 1.9e5 Ar (N = 5), 8.45 -> 8.07 on 1.7e5 H2 (N = 4); 6 spills: 17.6 and 9.0.
 // At N = 7 the stage derivatives (7 N doubles per thread) leave room for 4.
 template <int N>
@@ -366,8 +370,9 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
     // share of the electrons for each
     const long long all = (long long)gridDim.x * (kThreads / 32);
     const long long used = min(all, one_per_warp * ((n + 32ll * one_per_warp - 1) / (32ll * one_per_warp)));
-    if ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5) >= used) return;
+    if ((long long)blockIdx.x * (kThreads / 32) >= used) return;
     const int lanes = (int)min(32ll, (n + used - 1) / used);
+    const bool in_step = used > 2ll * one_per_warp;
     extern __shared__ double s_K[];
     double* const K = s_K + threadIdx.x;
     auto slot = [&](int l, int j) -> double& { return K[(l * N + j) * kThreads]; };
@@ -378,7 +383,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
 
     enum { kFree, kBase, kInit, kWait, kStep };
     int mode = kFree;
-    bool drained = false;
+    bool drained = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5) >= used;
     long long s = 0, g = 0;
     double u[N], w[N];  // accepted state; state to evaluate (at st = 6: the new state)
     double Fx = 0.0, Fy = 0.0, tl = 0.0, d1 = 0.0, r2min = 0.0;
@@ -397,6 +402,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
     };
 
     for (int st = 1;; st = (st == 6) ? 1 : st + 1) {
+        if (in_step && st != 1) __syncthreads();
         if (st == 1) {
             const bool had = mode != kFree;
             if (mode == kWait) mode = kStep;
@@ -435,8 +441,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
                     }
                 }
             }
-            if (__ballot_sync(FULL, mode != kFree) == 0u) break;
-            if (drained) {
+            if (drained && __ballot_sync(FULL, mode != kFree) != 0u) {
                 // the queue is empty: once few electrons are left in all, the others go to
                 // the second kernel, which has no use for full warps
                 unsigned long long fin = 0ull;
@@ -455,9 +460,10 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
                         for (int j = 0; j < N; ++j) store_component<DIM, PHASE>(soa, out, g, s, j, u[j]);
                         mode = kFree;
                     }
-                    if (__ballot_sync(FULL, mode != kFree) == 0u) break;
                 }
             }
+            // (in step, the block leaves together)
+            if (!(in_step ? __syncthreads_or(mode != kFree) != 0 : __ballot_sync(FULL, mode != kFree) != 0u)) break;
         }
         // ---- this turn's evaluation -----------------------------------------------------------
         if (mode == kStep) {
@@ -481,7 +487,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
         } else {
             tl = (mode == kInit) ? c.t + c.dt : c.t;
         }
-        if (mode == kFree || mode == kWait) continue;
+        if (mode == kFree || mode == kWait) continue;  // (to the barrier)
         if (!(mode == kStep && st == 6)) laser_F(J.laser, tl, Fx, Fy);  // stage 7 is at stage 6's time
         double du[N];
         rhs_at<DIM, PHASE, TGT>(J, Fx, Fy, w, du);

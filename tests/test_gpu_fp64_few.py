@@ -53,3 +53,17 @@ def test_whole_jobs_use_the_same_values(eng, dim, phase):
         fin, status, counts = eng.integrate(job, init)
         assert np.array_equal(counts, steps) and np.array_equal(status, st & 0xff)
         assert np.all(rmin <= np.sqrt((init[:, :dim] ** 2).sum(axis=1)) * (1 + 1e-15)) and np.all(rmin > 0)
+
+
+@pytest.mark.parametrize("dim,phase,target", [(2, "SCTS", "Ar"), (3, "QTMC", "H")])
+def test_electron_counts_around_blocks_in_step(eng, dim, phase, target):
+    """Up to two warps per sub-partition (38,912 electrons on 152 SMs) the first kernel's warps
+    run freely, above that a block's go in step; 97,281 are one more than all its lanes."""
+    job = job_of(method="SPANE", dim=dim, phase=phase, target=target, nt=60, nkd=21, nkz=5, laser="cos2",
+                 ellip=1.0 if dim == 2 else 0.5)
+    init = O.sample_all(job)
+    ref, rs, rn = O.integrate(job, init)
+    for n in (38912, 38913, 97281):
+        k = np.arange(n) % len(init)
+        fin, st, steps = eng.integrate(job, init[k])
+        assert np.array_equal(fin, ref[k]) and np.array_equal(st, rs[k]) and np.array_equal(steps, rn[k]), n
