@@ -118,11 +118,12 @@ INTEGRATOR_DRAM_BYTES_PER_ELECTRON = 30.48
 # main; 68 % FADD, 21 % FFMA, 8 % FMUL) per step attempt, and DRAM bytes (read +
 # write, 14.53 MB + 16.04 MB) per electron.  At that size the carry buffer between
 # the passes (116 B per electron) stays in L2; at full size it adds about that much
-# per electron again.  FMA-pipe issue (sm__inst_executed_pipe_fma, warp
-# instructions against 4 per SM and cycle) was 35.3 % (start-up) and 41.5 % (main).
+# per electron again.  Counted before the x and y components shared instructions: an
+# operation on a pair counts two.  FMA pipe: share of the cycles in which it is busy
+# (sm__pipe_fma_cycles_active; such an instruction takes it for two).
 DF_FP32_INST_PER_STEP = 6717
 DF_DRAM_BYTES_PER_ELECTRON = 189.0
-DF_FMA_PIPE_ISSUE_NCU = {"start_up": 0.348, "main": 0.505}
+DF_FMA_PIPE_ISSUE_NCU = {"start_up": 0.387, "main": 0.568}
 
 
 def rank_env():
