@@ -402,7 +402,10 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
     };
 
     for (int st = 1;; st = (st == 6) ? 1 : st + 1) {
-        if (in_step && st != 1) __syncthreads();
+        if (in_step && st != 1) {
+            __syncwarp();  // (lanes without an evaluation left the turn early)
+            __syncthreads();
+        }
         if (st == 1) {
             const bool had = mode != kFree;
             if (mode == kWait) mode = kStep;
