@@ -151,7 +151,7 @@ DFS_HD void table_piece(const DLaser& L, double T0, double h, int k, const DfTab
                                     {1, 0, -8, 0, 8, 0, 0, 0},      {0, 5, 0, -20, 0, 16, 0, 0},
                                     {-1, 0, 18, 0, -48, 0, 32, 0}, {0, -7, 0, 56, 0, -112, 0, 64}};
     double fx[8], fy[8];
-    for (int j = 0; j < 8; ++j) laser_F(L, T0 + h * ((double)k + 0.5 * (N.u[j] + 1.0)), fx[j], fy[j]);
+    for (int j = 0; j < 8; ++j) laser_F<false>(L, T0 + h * ((double)k + 0.5 * (N.u[j] + 1.0)), fx[j], fy[j]);
     double cx[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cy[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int m = 0; m < 8; ++m) {
         double ax = 0.0, ay = 0.0;

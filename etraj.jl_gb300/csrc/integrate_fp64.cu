@@ -491,7 +491,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
             tl = (mode == kInit) ? c.t + c.dt : c.t;
         }
         if (mode == kFree || mode == kWait) continue;  // (to the barrier)
-        if (!(mode == kStep && st == 6)) laser_F(J.laser, tl, Fx, Fy);  // stage 7 is at stage 6's time
+        if (!(mode == kStep && st == 6)) laser_F<false>(J.laser, tl, Fx, Fy);  // stage 7 is at stage 6's time
         double du[N];
         rhs_at<DIM, PHASE, TGT>(J, Fx, Fy, w, du);
         if (mode == kStep) {
@@ -659,7 +659,7 @@ k_integrate_fp64_few(const __grid_constant__ DJob J, InitSoA soa, const double* 
                 clock_start(c, t0, tf, lq0);
                 if (out.rmin) r2min = r2_of(u);
             }
-            laser_F(J.laser, c.t, Fx, Fy);
+            laser_F<false>(J.laser, c.t, Fx, Fy);
             K0 = rhs_of(Fx, Fy, u);
             if (!resume) {
                 const double sk = fma(fabs(u), J.rtol, ABSTOL);
@@ -668,7 +668,7 @@ k_integrate_fp64_few(const __grid_constant__ DJob J, InitSoA soa, const double* 
                 if (dt0 < 10.0 * 2.220446049250313e-16) {
                     c.dt = 1e-6;
                 } else {
-                    laser_F(J.laser, t0 + dt0, Fx, Fy);
+                    laser_F<false>(J.laser, t0 + dt0, Fx, Fy);
                     const double f1 = rhs_of(Fx, Fy, fma(dt0, K0, u));
                     c.dt = start_dt(d1, DM_DIV(rms_of<N>(sum_squares(DM_DIV(f1 - K0, sk))), dt0), dt0, c.dtmax, c.dtmin);
                 }
@@ -702,7 +702,7 @@ k_integrate_fp64_few(const __grid_constant__ DJob J, InitSoA soa, const double* 
         // the laser at the five stage times, one per lane
         const int m = lane & 7;
         double fx, fy;
-        laser_F(J.laser, (m < 4) ? fma(cC[m + 1], c.dt, c.t) : c.t + c.dt, fx, fy);
+        laser_F<false>(J.laser, (m < 4) ? fma(cC[m + 1], c.dt, c.t) : c.t + c.dt, fx, fy);
         // (a loop over the stages, its derivatives selected by index, is smaller code and was
         // slower: 5.4 against 5.0 ms on 1248 electrons)
         double K1, K2, K3, K4, K5, K6, w, a;

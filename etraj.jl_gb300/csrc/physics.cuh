@@ -24,13 +24,16 @@ __host__ __device__ __forceinline__ void window(const DMono& L, double tt, doubl
     w2 = 0.5 + 0.5 * dm_tanh(-L.k * (tt - L.Npiw));
 }
 
-// LaserFx / LaserFy of one monochromatic laser.
+// LaserFx / LaserFy of one monochromatic laser.  ZERO_SIGN: outside a cos^n pulse the field
+// is a zero whose sign is the carrier's.  The sampler takes a direction from it (atan2); an
+// equation of motion only adds it to the force, so there +0 serves and nothing is evaluated.
+template <bool ZERO_SIGN>
 __host__ __device__ __forceinline__ void mono_F(const DMono& L, double t, double& Fx, double& Fy) {
     double tt = t - L.t_shift;
     double sth, cth, pre, cx, cy;
 #if DM_INT
     const uint32_t at = fi_hi(tt) & 0x7fffffffu;
-    if (L.kind != ETRAJ_LASER_GAUSSIAN && at >= L.out_hi) { // after (or before) the pulse
+    if (!ZERO_SIGN && L.kind != ETRAJ_LASER_GAUSSIAN && at >= L.out_hi) { // after (or before) the pulse
         Fx = Fy = (tt != tt) ? tt : 0.0;
         return;
     }
@@ -68,11 +71,12 @@ __host__ __device__ __forceinline__ void mono_F(const DMono& L, double t, double
     }
 }
 
+template <bool ZERO_SIGN = true>
 __host__ __device__ __forceinline__ void laser_F(const DLaser& L, double t, double& Fx, double& Fy) {
-    mono_F(L.m[0], t, Fx, Fy);
+    mono_F<ZERO_SIGN>(L.m[0], t, Fx, Fy);
     if (L.nmono == 2) {
         double fx2, fy2;
-        mono_F(L.m[1], t - L.delay, fx2, fy2);
+        mono_F<ZERO_SIGN>(L.m[1], t - L.delay, fx2, fy2);
         Fx = Fx + fx2;
         Fy = Fy + fy2;
     }
