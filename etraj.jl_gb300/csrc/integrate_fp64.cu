@@ -471,6 +471,7 @@ k_integrate_fp64(const __grid_constant__ DJob J, InitSoA soa, const double* __re
                     }
                 }
             }
+            __syncwarp();  // (some lanes just handed an electron over, or took one)
             // (in step, the block leaves together)
             if (!(in_step ? __syncthreads_or(mode != kFree) != 0 : __ballot_sync(FULL, mode != kFree) != 0u)) break;
         }
