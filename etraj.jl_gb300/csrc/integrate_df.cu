@@ -208,6 +208,13 @@ k_integrate_df(const __grid_constant__ DFParams P, InitSoA soa, const double* __
                         mode = kBase;
                     }
                 }
+            } else if (MAIN && !drained) {
+                // a full warp has nothing to ask the queue for, and looks at it, so that its last
+                // electrons can leave too (32 slow ones: a call of 52 -> 32 ms); every 16th attempt
+                // of its first lane, as the block waits for the answer
+                unsigned long long taken = 0ull;
+                if (lane == 0 && (L.attempts & 15) == 0) taken = *(volatile unsigned long long*)queue;
+                drained = __shfl_sync(FULL, taken, 0) >= n_traj;
             }
             if (!__syncthreads_or(mode != kFree)) break;  // the block leaves together
         }
