@@ -287,7 +287,7 @@ int gather_rows(etraj_ctx* ctx, const HostJob& H, const Pipeline& P, int64_t g0,
         const int64_t chunks = (n + chunk - 1) / chunk;
         auto len = [&](int64_t c) { return std::min(chunk, n - c * chunk); };
         auto write = [&](int64_t c) {
-            launch_gather_rows(J, P.soa, P.t, P.idx, g0, c * chunk, len(c), (double*)blk[c & 1].p, s);
+            launch_gather_rows(J, P.soa, P.t, P.idx, g0, c * chunk, len(c), (double*)blk[c & 1].p, ctx->sm_count, s);
             cudaEventRecord(done[c & 1], s);
         };
         write(0);

@@ -195,7 +195,7 @@ int launch_compact(const uint8_t* flag, int64_t n, int64_t* idx, uint32_t* block
 int64_t compact_blocks(int64_t n);
 // Columns k0 .. k0 + n of the reference's `init` (J.rows doubles each): survivors g0 + idx[k].
 int launch_gather_rows(const DJob& J, const InitSoA& soa, const double* t, const int64_t* idx, int64_t g0, int64_t k0,
-                       int64_t n, double* out, cudaStream_t s);
+                       int64_t n, double* out, int sm_count, cudaStream_t s);
 // FP64 Tsit5 solve of the survivors; work: four counters.  Without out.final_state the
 // final states replace the initial ones in soa (a 3D z goes to out.c_im), where
 // launch_collect_fp64 reads them.

@@ -735,9 +735,9 @@ int launch_sample_range(const DJob& J, int64_t b0, int64_t nb, const double* kd,
 }
 
 int launch_gather_rows(const DJob& J, const InitSoA& soa, const double* t, const int64_t* idx, int64_t g0, int64_t k0,
-                       int64_t n, double* out, cudaStream_t s) {
-    const int64_t want = (n * J.rows + 255) / 256;
-    k_gather_rows<<<(unsigned)(want < 152 * 16 ? want : 152 * 16), 256, 0, s>>>(soa, t, idx, g0, k0, n, J.rows, J.dim, out);
+                       int64_t n, double* out, int sm_count, cudaStream_t s) {
+    const int64_t want = (n * J.rows + 255) / 256, cap = (int64_t)sm_count * 16;
+    k_gather_rows<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(soa, t, idx, g0, k0, n, J.rows, J.dim, out);
     return 1;
 }
 
