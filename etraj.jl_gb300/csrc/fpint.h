@@ -103,7 +103,8 @@ FI_FN uint32_t fi_mulhi(uint32_t a, uint32_t b) {
     return (uint32_t)(((uint64_t)a * b) >> 32);
 #endif
 }
-/* approximate 1/f and 1/sqrt(f), to 2^-22; FI_TEST_ERR moves the host's by that many ulp */
+/* approximate 1/f and 1/sqrt(f), off by at most 2^-23 and 2^-22.9 of them (the PTX
+ * manual's bounds); FI_TEST_ERR moves the host's by that many 2^-23 */
 FI_FN float fi_rcp_approx(float f) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -130,9 +131,11 @@ FI_FN float fi_rsqrt_approx(float f) {
 FI_FN uint64_t fi_mul64(uint32_t d, uint64_t m) {
     return (uint64_t)d * (uint32_t)m + ((uint64_t)(d * (uint32_t)(m >> 32)) << 32);
 }
-/* an approximation v of a reciprocal in [1/2, 1] as 2^32 v, lowered by 8 x 2^-24: with the
- * input's truncation (2 x 2^-24) and the approximation's error (2 x 2^-24) it is below
- * the true value by at most 2^-19.4 of it, and never above */
+/* an approximation v of a reciprocal in [1/2, 1] as 2^32 v, lowered by 8 x 2^-24.  The
+ * input's truncation raises v by at most 2 x 2^-24 (1/f) or 1 x 2^-24 (1/sqrt f), the
+ * approximation moves it by at most 2 x 2^-24 or 2.2 x 2^-24, so the result is never above
+ * the true value and below it by at most 10.2 x 2^-24, 2^-19.6 of it; the digits below allow
+ * 2^-19.4.  (The tests keep every bit at twice the approximations' errors.) */
 FI_FN uint32_t fi_below(float v) { return (fi_fbits(v) - 0x3f000000u - 8u) * 256u + 0x80000000u; }
 
 /* ---- a / b ---------------------------------------------------------------------
