@@ -111,19 +111,37 @@ FLOPS_PER_STEP_SAE_2D_SCTS = 702
 # this workload, from one ncu capture of a 2e6-candidate case (24.91 MB for 8.17e5
 # electrons); traffic grows with the electrons.
 INTEGRATOR_DRAM_BYTES_PER_ELECTRON = 30.48
-# The double-float integrator (start-up and main pass) on the same workload, from one
-# ncu capture of both passes on a 4e5-candidate case (400 time samples: 161,722
-# electrons, 6,489,343 step attempts): FP32 thread instructions
-# (smsp__sass_thread_inst_executed_op_fp32_pred_on: 4.07e9 start-up + 3.928e10
-# main; 68 % FADD, 21 % FFMA, 8 % FMUL) per step attempt, and DRAM bytes (read +
-# write, 14.53 MB + 16.04 MB) per electron.  At that size the carry buffer between
-# the passes (116 B per electron) stays in L2; at full size it adds about that much
-# per electron again.  Counted before the x and y components shared instructions: an
-# operation on a pair counts two.  FMA pipe: share of the cycles in which it is busy
-# (sm__pipe_fma_cycles_active; such an instruction takes it for two).
-DF_FP32_INST_PER_STEP = 6717
-DF_DRAM_BYTES_PER_ELECTRON = 189.0
-DF_FMA_PIPE_ISSUE_NCU = {"start_up": 0.387, "main": 0.568}
+# The double-float integrator on the same workload, from one ncu capture of its three
+# kernels on a 4e5-candidate case (400 time samples: 161,722 electrons, 6,489,343 step
+# attempts).  FP32 operations executed per step attempt, an operation on a pair counted
+# twice (smsp__sass_thread_inst_executed_op_fp32_pred_on, in which a pair's instruction is
+# one, plus its fadd2 and ffma2 parts): 4.05e9 in the start-up pass + 4.06e10 in the main
+# pass.  The third kernel's 6.8e8 are left out: its eight lanes repeat the target's terms.
+# DRAM bytes (read + write) per electron, all three: 16.1 + 16.0 + 2.3 MB.  At that size the
+# carry buffer between the passes (116 B per electron) stays in L2; at full size it adds
+# about that much per electron again.
+DF_FP32_OPS_PER_STEP = 6884
+DF_DRAM_BYTES_PER_ELECTRON = 213.0
+# FMA pipe in the same capture, two quantities.  issue: its warp instructions against the
+# four per SM and cycle that can be issued (sm__inst_executed_pipe_fma); an operation on a
+# pair is one instruction.  busy: the cycles in which the pipe works
+# (sm__pipe_fma_cycles_active); such an instruction takes it for two.
+DF_FMA_PIPE_ISSUE_NCU = {"start_up": 0.325, "main": 0.393, "few": 0.229}
+DF_FMA_PIPE_BUSY_NCU = {"start_up": 0.386, "main": 0.562, "few": 0.276}
+
+
+def df_roofline(attempts, kern_ms, electrons, n_sm, sm_max, headline):
+    """Roofline record of the double-float integrator (all three kernels): operations per
+    second against one FP32 operation per lane and cycle."""
+    ops = attempts * DF_FP32_OPS_PER_STEP / (kern_ms / 1e3) / 1e12 if (kern_ms and headline) else None
+    return {"bound": "fp32_issue", "achieved": ops, "peak": n_sm * 128 * sm_max * 1e6 / 1e12,
+            "unit": "T FP32 operations/s (an FMA is one, an operation on a pair two)",
+            "traffic": DF_DRAM_BYTES_PER_ELECTRON * electrons if headline else None,
+            "kernel": "k_integrate_df (start-up pass, main pass) and k_integrate_df_few", "kernel_ms": kern_ms,
+            "fp32_ops_per_step_attempt": DF_FP32_OPS_PER_STEP, "step_attempts_per_job": attempts,
+            "fma_pipe_issue_frac_ncu": DF_FMA_PIPE_ISSUE_NCU, "fma_pipe_busy_frac_ncu": DF_FMA_PIPE_BUSY_NCU,
+            "peak_source": "nominal FP32 issue: %d SMs x 128 lanes x %d MHz (no measured FP32 "
+                           "peak is provided)" % (n_sm, sm_max)}
 
 
 def rank_env():
@@ -400,19 +418,7 @@ def main():
         steps_per_job = steps_total / args.steps
         eff_mean = statistics.mean(effs)
         if args.precision == "fp32_df":
-            # FP32-pipe issue: thread instructions per second against 128 lanes x SMs x clock
-            per_step = DF_FP32_INST_PER_STEP
-            achieved = (steps_per_job * per_step / (kern_ms / 1e3) / 1e12
-                        if (kern_ms and headline and per_step) else None)
-            roof = {"bound": "fp32_issue", "achieved": achieved, "peak": n_sm * 128 * sm_max * 1e6 / 1e12,
-                    "unit": "T FP32-pipe thread instructions/s",
-                    "traffic": (DF_DRAM_BYTES_PER_ELECTRON * eff_mean)
-                    if (headline and DF_DRAM_BYTES_PER_ELECTRON) else None,
-                    "kernel": "k_integrate_df (start-up + main pass)", "kernel_ms": kern_ms,
-                    "fp32_inst_per_step_attempt": per_step, "step_attempts_per_job": steps_per_job,
-                    "fma_pipe_issue_frac_ncu": DF_FMA_PIPE_ISSUE_NCU,
-                    "peak_source": "nominal FP32 issue: %d SMs x 128 lanes x %d MHz (no measured FP32 "
-                                   "peak is provided)" % (n_sm, sm_max)}
+            roof = df_roofline(steps_per_job, kern_ms, eff_mean, n_sm, sm_max, headline)
         else:
             flops = steps_per_job * FLOPS_PER_STEP_SAE_2D_SCTS
             # the flop count per step is the headline workload's (2D SAE SCTS)
