@@ -484,8 +484,10 @@ def accuracy_report(eng, job, job64, job_other=None):
     """PMD error of the timed path against the FP64 plain path on the same electrons,
     next to the FP64 path's own sensitivity to its tolerance (rtol 1e-6 vs 1e-7), at
     the full 1000 x 1000 resolution and after rebinning to 100 x 100 and 20 x 20;
-    job_other (the other FP32 path) gets its speed (5 runs) and PMD error beside it."""
+    job_other (the other FP32 path) gets its speed (5 runs) and PMD error beside it.  The
+    FP64 path's time is the least of three runs after the first, which loads its kernels (15 ms)."""
     res64, spec64, _ = eng.run(job64, want_spectrum=True)
+    ms64 = min(eng.run(job64, want_spectrum=False)[0].elapsed_ms for _ in range(3))
     res, spec, _ = eng.run(job, want_spectrum=True)
     j7 = job64.copy()
     j7.traj_rtol = 1e-7
@@ -504,8 +506,8 @@ def accuracy_report(eng, job, job64, job_other=None):
                 a = np.add.reduceat(a, np.arange(0, a.shape[ax], f), axis=ax)
         return a.ravel()
 
-    out = {"fp64_plain": {"value": res64.num_effective_traj / (res64.elapsed_ms / 1e3), "unit": UNIT,
-                          "ms_per_step": res64.elapsed_ms},
+    out = {"fp64_plain": {"value": res64.num_effective_traj / (ms64 / 1e3), "unit": UNIT,
+                          "ms_per_step": ms64},
            "pmd_rel_l2_vs_fp64": l2(spec, spec64),
            "fp64_rtol1e-7_vs_rtol1e-6_pmd_rel_l2": l2(spec64b, spec64),
            "ion_prob_rel_diff": abs(res.ion_prob - res64.ion_prob) / res64.ion_prob}
@@ -523,7 +525,7 @@ def accuracy_report(eng, job, job64, job_other=None):
         out[name] = {
             "value": r.num_effective_traj / (min(ms) / 1e3), "unit": UNIT, "ms_per_step": min(ms),
             "pmd_rel_l2_vs_fp64": l2(so, spec64), "pmd_rel_l2_vs_fp64_rebin50": l2(rebin(so, 50), rebin(spec64, 50)),
-            "speedup_vs_fp64": res64.elapsed_ms / min(ms)}
+            "speedup_vs_fp64": ms64 / min(ms)}
     return out
 
 
