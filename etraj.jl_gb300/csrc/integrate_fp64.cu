@@ -21,8 +21,9 @@
 // are two kernels for two loads:
 //  * k_integrate_fp64, many electrons: one per lane, so a warp instruction serves 32.
 //    Persistent; a lane that finishes takes the next electron from a queue, so step
-//    counts that differ within a warp do not idle it.  ~500 FP64 instructions per
-//    attempt and warp.
+//    counts that differ within a warp do not idle it.  FP64 operations per
+//    attempt, so warp instructions of a full warp: 470 to 500 (hydrogen-like, 2D), 750 (an
+//    SAE atom with a phase, 2D), 920 (3D).
 //  * k_integrate_fp64_few, few electrons: eight lanes each.  The laser at an attempt's
 //    five stage times (it does not depend on the state), the components' stage and
 //    error sums and the controller's two powers run in parallel lanes: ~180 FP64
