@@ -506,7 +506,14 @@ int enqueue_job(etraj_ctx* ctx, const etraj_job* job, JobRec& r) {
     cudaMemcpyAsync(dst_sums, P.sums, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(dst_cnt, P.counters, sizeof(Counters), cudaMemcpyDeviceToHost, s);
     if (dst_spec) cudaMemcpyAsync(dst_spec, P.mspec, (size_t)J.grid * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (dst_amp) cudaMemcpyAsync(dst_amp, P.spec, (size_t)J.grid * 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (dst_amp && r.coherent) {
+        cudaMemcpyAsync(dst_amp, P.spec, (size_t)J.grid * 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
+    } else if (dst_amp) {
+        // a CTMC job's sums are real, one double a bin
+        for (int64_t k = 0; k < J.grid; ++k) dst_amp[2 * k + 1] = 0.0;
+        cudaMemcpy2DAsync(dst_amp, 2 * sizeof(double), P.spec, sizeof(double), sizeof(double), (size_t)J.grid,
+                          cudaMemcpyDeviceToHost, s);
+    }
     cudaEventRecord(r.ev_done, s);
     r.launches = launches;
     cudaError_t e = cudaGetLastError();
