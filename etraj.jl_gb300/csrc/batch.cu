@@ -319,8 +319,8 @@ int sample_range(etraj_ctx* ctx, const etraj_job* job, int64_t b0, int64_t nb, d
     prepare_job(job, H);
     Pipeline P;
     ETRAJ_TRY(alloc_sampling(ctx, H, P));
-    // (a count of its own: the jobs' still tells how many states a dump of the last one has)
-    ETRAJ_TRY(ensure_t(ctx, "sample.count", 4, &P.count));
+    // (the second of its four counts: the first tells how many states a dump of the last job has)
+    P.count += 1;
     cudaStream_t s = ctx->stream;
     upload_inputs(H, P, s);
     launch_batch_prepare(H.J, P.t, P.batches, s);
